@@ -6,12 +6,13 @@
 // the API unchanged.  Values are kept fully reduced in [0, m).
 //
 // Multiplication is separated Montgomery with 32-bit limbs: the 512-bit
-// product comes from one level of Karatsuba over 128-bit halves (three 4 x 4
-// limb schoolbook products, 96 multiply instructions instead of 128), then
-// eight reduction rows against the modulus, whose limbs are PTX immediates,
-// fold the low half and the high half is added at the end.  Each schoolbook
-// or reduction row is two interleaved carry chains (even / odd limb
-// products, mad.lo/madc.hi).  Both BN254 moduli are below 2^254, which bounds
+// product first (schoolbook, 64 multiply pairs), then eight reduction rows
+// against the modulus, whose limbs are PTX immediates, fold the low half and
+// the high half is added at the end.  Every sum of limb products is kept in
+// two accumulators by the parity of the limb position, so that each
+// mad.lo/madc.hi pair is one aligned 64-bit multiply-add.  The unreduced
+// products also enter sums of products with one reduction (Fp2 products,
+// differences).  Both BN254 moduli are below 2^254, which bounds
 // every intermediate (derivations at the functions).  The products are
 // bit-identical to the reference's 4 x u64 CIOS fpMul / frMul
 // (include/fp_bn254.cuh:187-277, include/fr_bn254.cuh:173-210): both return
@@ -183,279 +184,271 @@ __device__ __forceinline__ fe<C> fe_dbl(const fe<C>& a) {
 }
 
 // ------------------------------------------------------------------- mul
-// t += m * modulus, modulus limbs as immediates
-#define ZK_RED_EVEN(M)                                                                      \
-  asm("mad.lo.cc.u32  %0, %13, %9, %0;\n\t"                                                 \
-      "madc.hi.cc.u32 %1, %13, %9, %1;\n\t"                                                 \
-      "madc.lo.cc.u32 %2, %13, %10, %2;\n\t"                                                \
-      "madc.hi.cc.u32 %3, %13, %10, %3;\n\t"                                                \
-      "madc.lo.cc.u32 %4, %13, %11, %4;\n\t"                                                \
-      "madc.hi.cc.u32 %5, %13, %11, %5;\n\t"                                                \
-      "madc.lo.cc.u32 %6, %13, %12, %6;\n\t"                                                \
-      "madc.hi.cc.u32 %7, %13, %12, %7;\n\t"                                                \
-      "addc.u32       %8, %8, 0;"                                                           \
-      : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), \
-        "+r"(t8)                                                                            \
-      : "n"(C::P0), "n"(C::P2), "n"(C::P4), "n"(C::P6), "r"(M))
-#define ZK_RED_ODD(M)                                                                       \
-  asm("mad.lo.cc.u32  %0, %12, %8, %0;\n\t"                                                 \
-      "madc.hi.cc.u32 %1, %12, %8, %1;\n\t"                                                 \
-      "madc.lo.cc.u32 %2, %12, %9, %2;\n\t"                                                 \
-      "madc.hi.cc.u32 %3, %12, %9, %3;\n\t"                                                 \
-      "madc.lo.cc.u32 %4, %12, %10, %4;\n\t"                                                \
-      "madc.hi.cc.u32 %5, %12, %10, %5;\n\t"                                                \
-      "madc.lo.cc.u32 %6, %12, %11, %6;\n\t"                                                \
-      "madc.hi.u32    %7, %12, %11, %7;"                                                    \
-      : "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)      \
-      : "n"(C::P1), "n"(C::P3), "n"(C::P5), "n"(C::P7), "r"(M))
-
-// r[0..7] = x[0..3] * y[0..3].  Row j adds x * y_j at limb j as an even
-// chain (x0, x2) that also produces limb j+4 and an odd chain (x1, x3) that
-// ends there: the partial product after row j is below 2^(32(j+5)), so the
-// odd chain's last madc.hi never carries out.  Outputs are early-clobber:
-// they are written while inputs are still being read.
-__device__ __forceinline__ void mul_4x4(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3,
-                                        uint32_t y0, uint32_t y1, uint32_t y2, uint32_t y3,
-                                        uint32_t (&r)[8]) {
-  asm("mul.lo.u32     %0, %8, %12;\n\t"
-      "mul.hi.u32     %1, %8, %12;\n\t"
-      "mul.lo.u32     %2, %10, %12;\n\t"
-      "mul.hi.u32     %3, %10, %12;\n\t"
-      "mad.lo.cc.u32  %1, %9, %12, %1;\n\t"
-      "madc.hi.cc.u32 %2, %9, %12, %2;\n\t"
-      "madc.lo.cc.u32 %3, %11, %12, %3;\n\t"
-      "madc.hi.u32    %4, %11, %12, 0;\n\t"
-      "mad.lo.cc.u32  %1, %8, %13, %1;\n\t"
-      "madc.hi.cc.u32 %2, %8, %13, %2;\n\t"
-      "madc.lo.cc.u32 %3, %10, %13, %3;\n\t"
-      "madc.hi.cc.u32 %4, %10, %13, %4;\n\t"
-      "addc.u32       %5, 0, 0;\n\t"
-      "mad.lo.cc.u32  %2, %9, %13, %2;\n\t"
-      "madc.hi.cc.u32 %3, %9, %13, %3;\n\t"
+// Multiply-add chains on aligned word pairs.  A pair mad.lo.cc / madc.hi.cc
+// on an even-odd pair of accumulator words is one 64-bit multiply-add with
+// carry in the machine, at a quarter of the simple instructions' rate; pairs
+// that straddle the alignment cost moves or two instructions.  So every sum
+// of limb products keeps two accumulators: one for products whose position is
+// even, one for odd positions (stored a word lower), and adds them up at the
+// end.
+//
+// e[0..7] += (x0, x1, x2, x3 at words 0, 2, 4, 6) * y; the carry joins c.
+__device__ __forceinline__ void mac4(uint32_t* e, uint32_t& c, uint32_t x0, uint32_t x1,
+                                     uint32_t x2, uint32_t x3, uint32_t y) {
+  asm("mad.lo.cc.u32  %0, %9, %13, %0;\n\t"
+      "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+      "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+      "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
       "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
-      "madc.hi.u32    %5, %11, %13, %5;\n\t"
-      "mad.lo.cc.u32  %2, %8, %14, %2;\n\t"
-      "madc.hi.cc.u32 %3, %8, %14, %3;\n\t"
-      "madc.lo.cc.u32 %4, %10, %14, %4;\n\t"
-      "madc.hi.cc.u32 %5, %10, %14, %5;\n\t"
-      "addc.u32       %6, 0, 0;\n\t"
-      "mad.lo.cc.u32  %3, %9, %14, %3;\n\t"
-      "madc.hi.cc.u32 %4, %9, %14, %4;\n\t"
-      "madc.lo.cc.u32 %5, %11, %14, %5;\n\t"
-      "madc.hi.u32    %6, %11, %14, %6;\n\t"
-      "mad.lo.cc.u32  %3, %8, %15, %3;\n\t"
-      "madc.hi.cc.u32 %4, %8, %15, %4;\n\t"
-      "madc.lo.cc.u32 %5, %10, %15, %5;\n\t"
-      "madc.hi.cc.u32 %6, %10, %15, %6;\n\t"
-      "addc.u32       %7, 0, 0;\n\t"
-      "mad.lo.cc.u32  %4, %9, %15, %4;\n\t"
-      "madc.hi.cc.u32 %5, %9, %15, %5;\n\t"
-      "madc.lo.cc.u32 %6, %11, %15, %6;\n\t"
-      "madc.hi.u32    %7, %11, %15, %7;"
-      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]),
-        "=&r"(r[6]), "=&r"(r[7])
-      : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y0), "r"(y1), "r"(y2), "r"(y3));
+      "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+      "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+      "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+      "addc.u32       %8, %8, 0;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]),
+        "+r"(e[7]), "+r"(c)
+      : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y));
 }
-
-// r[0..7] = x[0..3]^2: the six cross products once (positions 1-2, 3-4,
-// 5-6 written directly, then x0 x2 + x1 x3 as one chain and x0 x3 as
-// another), doubled, plus the four squares on the diagonal: 20 multiply
-// instructions instead of 32.  The doubled cross sum is below 2^256.
-__device__ __forceinline__ void sqr_4x4(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3,
-                                        uint32_t (&r)[8]) {
-  asm("mul.lo.u32     %1, %8, %9;\n\t"
-      "mul.hi.u32     %2, %8, %9;\n\t"
-      "mul.lo.u32     %3, %9, %10;\n\t"
-      "mul.hi.u32     %4, %9, %10;\n\t"
-      "mul.lo.u32     %5, %10, %11;\n\t"
-      "mul.hi.u32     %6, %10, %11;\n\t"
-      "mad.lo.cc.u32  %2, %8, %10, %2;\n\t"
+// the same where no carry can leave word 7
+__device__ __forceinline__ void mac4_top(uint32_t* e, uint32_t x0, uint32_t x1, uint32_t x2,
+                                         uint32_t x3, uint32_t y) {
+  asm("mad.lo.cc.u32  %0, %8, %12, %0;\n\t"
+      "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
+      "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
+      "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
+      "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+      "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+      "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
+      "madc.hi.u32    %7, %11, %12, %7;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]),
+        "+r"(e[7])
+      : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y));
+}
+// shorter rows of the same
+__device__ __forceinline__ void mac3(uint32_t* e, uint32_t& c, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t y) {
+  asm("mad.lo.cc.u32  %0, %7, %10, %0;\n\t"
+      "madc.hi.cc.u32 %1, %7, %10, %1;\n\t"
+      "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
       "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
-      "madc.lo.cc.u32 %4, %9, %11, %4;\n\t"
-      "madc.hi.cc.u32 %5, %9, %11, %5;\n\t"
-      "addc.u32       %6, %6, 0;\n\t"
-      "mad.lo.cc.u32  %3, %8, %11, %3;\n\t"
-      "madc.hi.cc.u32 %4, %8, %11, %4;\n\t"
-      "addc.cc.u32    %5, %5, 0;\n\t"
-      "addc.cc.u32    %6, %6, 0;\n\t"
-      "addc.u32       %7, 0, 0;\n\t"
-      "add.cc.u32     %1, %1, %1;\n\t"
-      "addc.cc.u32    %2, %2, %2;\n\t"
-      "addc.cc.u32    %3, %3, %3;\n\t"
-      "addc.cc.u32    %4, %4, %4;\n\t"
-      "addc.cc.u32    %5, %5, %5;\n\t"
-      "addc.cc.u32    %6, %6, %6;\n\t"
-      "addc.u32       %7, %7, %7;\n\t"
-      "mul.lo.u32     %0, %8, %8;\n\t"
-      "mad.hi.cc.u32  %1, %8, %8, %1;\n\t"
-      "madc.lo.cc.u32 %2, %9, %9, %2;\n\t"
-      "madc.hi.cc.u32 %3, %9, %9, %3;\n\t"
-      "madc.lo.cc.u32 %4, %10, %10, %4;\n\t"
-      "madc.hi.cc.u32 %5, %10, %10, %5;\n\t"
-      "madc.lo.cc.u32 %6, %11, %11, %6;\n\t"
-      "madc.hi.u32    %7, %11, %11, %7;"
-      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]),
-        "=&r"(r[6]), "=&r"(r[7])
-      : "r"(x0), "r"(x1), "r"(x2), "r"(x3));
+      "madc.lo.cc.u32 %4, %9, %10, %4;\n\t"
+      "madc.hi.cc.u32 %5, %9, %10, %5;\n\t"
+      "addc.u32       %6, %6, 0;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(c)
+      : "r"(x0), "r"(x1), "r"(x2), "r"(y));
+}
+__device__ __forceinline__ void mac3_top(uint32_t* e, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t y) {
+  asm("mad.lo.cc.u32  %0, %6, %9, %0;\n\t"
+      "madc.hi.cc.u32 %1, %6, %9, %1;\n\t"
+      "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
+      "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
+      "madc.lo.cc.u32 %4, %8, %9, %4;\n\t"
+      "madc.hi.u32    %5, %8, %9, %5;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5])
+      : "r"(x0), "r"(x1), "r"(x2), "r"(y));
+}
+__device__ __forceinline__ void mac2(uint32_t* e, uint32_t& c, uint32_t x0, uint32_t x1, uint32_t y) {
+  asm("mad.lo.cc.u32  %0, %5, %7, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+      "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"
+      "addc.u32       %4, %4, 0;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(c)
+      : "r"(x0), "r"(x1), "r"(y));
+}
+__device__ __forceinline__ void mac2_top(uint32_t* e, uint32_t x0, uint32_t x1, uint32_t y) {
+  asm("mad.lo.cc.u32  %0, %4, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %6, %2;\n\t"
+      "madc.hi.u32    %3, %5, %6, %3;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3])
+      : "r"(x0), "r"(x1), "r"(y));
+}
+__device__ __forceinline__ void mac1(uint32_t* e, uint32_t& c, uint32_t x0, uint32_t y) {
+  asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+      "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+      "addc.u32       %2, %2, 0;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(c)
+      : "r"(x0), "r"(y));
+}
+__device__ __forceinline__ void mac1_top(uint32_t* e, uint32_t x0, uint32_t y) {
+  asm("mad.lo.cc.u32  %0, %2, %3, %0;\n\t"
+      "madc.hi.u32    %1, %2, %3, %1;"
+      : "+r"(e[0]), "+r"(e[1])
+      : "r"(x0), "r"(y));
+}
+// e[0], e[1] = x * y
+__device__ __forceinline__ void mul_pair(uint32_t* e, uint32_t x, uint32_t y) {
+  asm("mul.lo.u32 %0, %2, %3;\n\tmul.hi.u32 %1, %2, %3;" : "=&r"(e[0]), "=r"(e[1]) : "r"(x), "r"(y));
 }
 
-// T[0..15] = a^2 for a < 2^255: aL^2 + 2 aL aH 2^128 + aH^2 2^256
-// (20 + 32 + 20 = 72 multiply instructions instead of Karatsuba's 96).
-__device__ __forceinline__ void fe_sqr_wide(const uint32_t (&a)[8], uint32_t (&T)[16]) {
-  uint32_t lo[8], hi[8], x[8], x8;
-  sqr_4x4(a[0], a[1], a[2], a[3], lo);
-  sqr_4x4(a[4], a[5], a[6], a[7], hi);
-  mul_4x4(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], x);
-  asm("add.cc.u32  %0, %0, %0;\n\t"
-      "addc.cc.u32 %1, %1, %1;\n\t"
-      "addc.cc.u32 %2, %2, %2;\n\t"
-      "addc.cc.u32 %3, %3, %3;\n\t"
-      "addc.cc.u32 %4, %4, %4;\n\t"
-      "addc.cc.u32 %5, %5, %5;\n\t"
-      "addc.cc.u32 %6, %6, %6;\n\t"
-      "addc.cc.u32 %7, %7, %7;\n\t"
-      "addc.u32    %8, 0, 0;"
-      : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]),
-        "+r"(x[7]), "=r"(x8));
-  T[0] = lo[0]; T[1] = lo[1]; T[2] = lo[2]; T[3] = lo[3];
-  asm("add.cc.u32  %0, %12, %20;\n\t"
-      "addc.cc.u32 %1, %13, %21;\n\t"
-      "addc.cc.u32 %2, %14, %22;\n\t"
-      "addc.cc.u32 %3, %15, %23;\n\t"
-      "addc.cc.u32 %4, %16, %24;\n\t"
-      "addc.cc.u32 %5, %17, %25;\n\t"
-      "addc.cc.u32 %6, %18, %26;\n\t"
-      "addc.cc.u32 %7, %19, %27;\n\t"
-      "addc.cc.u32 %8, %29, %28;\n\t"
-      "addc.cc.u32 %9, %30, 0;\n\t"
-      "addc.cc.u32 %10, %31, 0;\n\t"
-      "addc.u32    %11, %32, 0;"
-      : "=r"(T[4]), "=r"(T[5]), "=r"(T[6]), "=r"(T[7]), "=r"(T[8]), "=r"(T[9]), "=r"(T[10]),
-        "=r"(T[11]), "=r"(T[12]), "=r"(T[13]), "=r"(T[14]), "=r"(T[15])
-      : "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]),
-        "r"(hi[3]), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]),
-        "r"(x[7]), "r"(x8), "r"(hi[4]), "r"(hi[5]), "r"(hi[6]), "r"(hi[7]));
+// T = E + O 2^32 (O[15] = 0; the caller's sum is below 2^512).
+__device__ __forceinline__ void merge_16(const uint32_t (&E)[16], const uint32_t (&O)[16],
+                                         uint32_t (&T)[16]) {
+  T[0] = E[0];
+  asm("add.cc.u32  %0, %15, %30;\n\t"
+      "addc.cc.u32 %1, %16, %31;\n\t"
+      "addc.cc.u32 %2, %17, %32;\n\t"
+      "addc.cc.u32 %3, %18, %33;\n\t"
+      "addc.cc.u32 %4, %19, %34;\n\t"
+      "addc.cc.u32 %5, %20, %35;\n\t"
+      "addc.cc.u32 %6, %21, %36;\n\t"
+      "addc.cc.u32 %7, %22, %37;\n\t"
+      "addc.cc.u32 %8, %23, %38;\n\t"
+      "addc.cc.u32 %9, %24, %39;\n\t"
+      "addc.cc.u32 %10, %25, %40;\n\t"
+      "addc.cc.u32 %11, %26, %41;\n\t"
+      "addc.cc.u32 %12, %27, %42;\n\t"
+      "addc.cc.u32 %13, %28, %43;\n\t"
+      "addc.u32    %14, %29, %44;"
+      : "=r"(T[1]), "=r"(T[2]), "=r"(T[3]), "=r"(T[4]), "=r"(T[5]), "=r"(T[6]), "=r"(T[7]),
+        "=r"(T[8]), "=r"(T[9]), "=r"(T[10]), "=r"(T[11]), "=r"(T[12]), "=r"(T[13]), "=r"(T[14]),
+        "=r"(T[15])
+      : "r"(E[1]), "r"(E[2]), "r"(E[3]), "r"(E[4]), "r"(E[5]), "r"(E[6]), "r"(E[7]), "r"(E[8]),
+        "r"(E[9]), "r"(E[10]), "r"(E[11]), "r"(E[12]), "r"(E[13]), "r"(E[14]), "r"(E[15]),
+        "r"(O[0]), "r"(O[1]), "r"(O[2]), "r"(O[3]), "r"(O[4]), "r"(O[5]), "r"(O[6]), "r"(O[7]),
+        "r"(O[8]), "r"(O[9]), "r"(O[10]), "r"(O[11]), "r"(O[12]), "r"(O[13]), "r"(O[14]));
 }
 
-// T[0..15] = a * b for a, b < 2^255 (one Karatsuba level over 128-bit
-// halves): T = lo + (mid - lo - hi) 2^128 + hi 2^256 with lo = aL bL,
-// hi = aH bH, mid = (aL + aH)(bL + bH).  The half sums are 129-bit (carry
-// bits ca, cb), so mid is the 4 x 4 product of their low limbs plus
-// (ca sb + cb sa) 2^128 + ca cb 2^256, kept in nine limbs (mid < 2^258).
-// Order keeps few values live: mid first, then lo folded into T[0..12], then
-// hi added at 2^256 and subtracted at 2^128.  Every partial sum is a
-// nonnegative part of the product (mid - lo >= hi), so no chain borrows out,
-// and the largest, a b + hi 2^128 < 2^510 + 2^382, fits in 16 limbs (inputs
-// near 2^256 would not: field elements and unreduced sums of two stay below
-// 2^255).
+// T[0..15] = a * b for any 256-bit a and b, schoolbook by rows of b: 64
+// multiply pairs.  After row j the sum of either parity is below
+// 2^(32 (j + 9)), so a row's odd-limb chain (whose last pair is the first to
+// reach its two words) ends without a carry and its even-limb chain carries
+// into a word that only a carry has reached before.
+// One Karatsuba level (48 pairs) saves a fifth of the pairs but adds ~100
+// instructions in sums and moves, a third of them on the multiply pipe: 62.9
+// against 61.5 G products/s at 32 warps per SM and equal at 8, with 294
+// against 228 instructions a product, which the kernels that are short of
+// issue slots or instruction cache pay for.
 __device__ __forceinline__ void fe_mul_wide(const uint32_t (&a)[8], const uint32_t (&b)[8],
                                             uint32_t (&T)[16]) {
-  uint32_t sa0, sa1, sa2, sa3, ca, sb0, sb1, sb2, sb3, cb;
-  asm("add.cc.u32  %0, %5, %9;\n\t"
-      "addc.cc.u32 %1, %6, %10;\n\t"
-      "addc.cc.u32 %2, %7, %11;\n\t"
-      "addc.cc.u32 %3, %8, %12;\n\t"
-      "addc.u32    %4, 0, 0;"
-      : "=r"(sa0), "=r"(sa1), "=r"(sa2), "=r"(sa3), "=r"(ca)
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
-  asm("add.cc.u32  %0, %5, %9;\n\t"
-      "addc.cc.u32 %1, %6, %10;\n\t"
-      "addc.cc.u32 %2, %7, %11;\n\t"
-      "addc.cc.u32 %3, %8, %12;\n\t"
-      "addc.u32    %4, 0, 0;"
-      : "=r"(sb0), "=r"(sb1), "=r"(sb2), "=r"(sb3), "=r"(cb)
-      : "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]));
-  uint32_t mid[8], m8;
-  mul_4x4(sa0, sa1, sa2, sa3, sb0, sb1, sb2, sb3, mid);
-  const uint32_t ma = 0u - ca, mb = 0u - cb;
-  asm("add.cc.u32  %0, %0, %5;\n\t"
-      "addc.cc.u32 %1, %1, %6;\n\t"
-      "addc.cc.u32 %2, %2, %7;\n\t"
-      "addc.cc.u32 %3, %3, %8;\n\t"
-      "addc.u32    %4, 0, 0;"
-      : "+r"(mid[4]), "+r"(mid[5]), "+r"(mid[6]), "+r"(mid[7]), "=r"(m8)
-      : "r"(sb0 & ma), "r"(sb1 & ma), "r"(sb2 & ma), "r"(sb3 & ma));
-  asm("add.cc.u32  %0, %0, %5;\n\t"
-      "addc.cc.u32 %1, %1, %6;\n\t"
-      "addc.cc.u32 %2, %2, %7;\n\t"
-      "addc.cc.u32 %3, %3, %8;\n\t"
-      "addc.u32    %4, %4, %9;"
-      : "+r"(mid[4]), "+r"(mid[5]), "+r"(mid[6]), "+r"(mid[7]), "+r"(m8)
-      : "r"(sa0 & mb), "r"(sa1 & mb), "r"(sa2 & mb), "r"(sa3 & mb), "r"(ca & cb));
-  // lo: T[0..12] = lo + (mid - lo) 2^128
-  uint32_t w[8];
-  mul_4x4(a[0], a[1], a[2], a[3], b[0], b[1], b[2], b[3], w);
-  asm("sub.cc.u32  %0, %0, %9;\n\t"
-      "subc.cc.u32 %1, %1, %10;\n\t"
-      "subc.cc.u32 %2, %2, %11;\n\t"
-      "subc.cc.u32 %3, %3, %12;\n\t"
-      "subc.cc.u32 %4, %4, %13;\n\t"
-      "subc.cc.u32 %5, %5, %14;\n\t"
-      "subc.cc.u32 %6, %6, %15;\n\t"
-      "subc.cc.u32 %7, %7, %16;\n\t"
-      "subc.u32    %8, %8, 0;"
-      : "+r"(mid[0]), "+r"(mid[1]), "+r"(mid[2]), "+r"(mid[3]), "+r"(mid[4]), "+r"(mid[5]),
-        "+r"(mid[6]), "+r"(mid[7]), "+r"(m8)
-      : "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]));
-  T[0] = w[0]; T[1] = w[1]; T[2] = w[2]; T[3] = w[3];
-  asm("add.cc.u32  %0, %9, %13;\n\t"
-      "addc.cc.u32 %1, %10, %14;\n\t"
-      "addc.cc.u32 %2, %11, %15;\n\t"
-      "addc.cc.u32 %3, %12, %16;\n\t"
-      "addc.cc.u32 %4, %17, 0;\n\t"
-      "addc.cc.u32 %5, %18, 0;\n\t"
-      "addc.cc.u32 %6, %19, 0;\n\t"
-      "addc.cc.u32 %7, %20, 0;\n\t"
-      "addc.u32    %8, %21, 0;"
-      : "=r"(T[4]), "=r"(T[5]), "=r"(T[6]), "=r"(T[7]), "=r"(T[8]), "=r"(T[9]), "=r"(T[10]),
-        "=r"(T[11]), "=r"(T[12])
-      : "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(mid[0]), "r"(mid[1]), "r"(mid[2]),
-        "r"(mid[3]), "r"(mid[4]), "r"(mid[5]), "r"(mid[6]), "r"(mid[7]), "r"(m8));
-  // hi: add at 2^256, subtract at 2^128
-  mul_4x4(a[4], a[5], a[6], a[7], b[4], b[5], b[6], b[7], w);
-  asm("add.cc.u32  %0, %0, %8;\n\t"
-      "addc.cc.u32 %1, %1, %9;\n\t"
-      "addc.cc.u32 %2, %2, %10;\n\t"
-      "addc.cc.u32 %3, %3, %11;\n\t"
-      "addc.cc.u32 %4, %4, %12;\n\t"
-      "addc.cc.u32 %5, %13, 0;\n\t"
-      "addc.cc.u32 %6, %14, 0;\n\t"
-      "addc.u32    %7, %15, 0;"
-      : "+r"(T[8]), "+r"(T[9]), "+r"(T[10]), "+r"(T[11]), "+r"(T[12]), "=r"(T[13]), "=r"(T[14]),
-        "=r"(T[15])
-      : "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]));
-  asm("sub.cc.u32  %0, %0, %12;\n\t"
-      "subc.cc.u32 %1, %1, %13;\n\t"
-      "subc.cc.u32 %2, %2, %14;\n\t"
-      "subc.cc.u32 %3, %3, %15;\n\t"
-      "subc.cc.u32 %4, %4, %16;\n\t"
-      "subc.cc.u32 %5, %5, %17;\n\t"
-      "subc.cc.u32 %6, %6, %18;\n\t"
-      "subc.cc.u32 %7, %7, %19;\n\t"
-      "subc.cc.u32 %8, %8, 0;\n\t"
-      "subc.cc.u32 %9, %9, 0;\n\t"
-      "subc.cc.u32 %10, %10, 0;\n\t"
-      "subc.u32    %11, %11, 0;"
-      : "+r"(T[4]), "+r"(T[5]), "+r"(T[6]), "+r"(T[7]), "+r"(T[8]), "+r"(T[9]), "+r"(T[10]),
-        "+r"(T[11]), "+r"(T[12]), "+r"(T[13]), "+r"(T[14]), "+r"(T[15])
-      : "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]));
+  uint32_t E[16], O[16];
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    mul_pair(E + i, a[i], b[0]);
+    mul_pair(O + i, a[i + 1], b[0]);
+  }
+#pragma unroll
+  for (int i = 8; i < 16; i++) E[i] = O[i] = 0;
+#pragma unroll
+  for (int j = 1; j < 8; j += 2) {
+    mac4(O + j - 1, O[j + 7], a[0], a[2], a[4], a[6], b[j]);
+    mac4_top(E + j + 1, a[1], a[3], a[5], a[7], b[j]);
+    if (j < 7) {
+      mac4(E + j + 1, E[j + 9], a[0], a[2], a[4], a[6], b[j + 1]);
+      mac4_top(O + j + 1, a[1], a[3], a[5], a[7], b[j + 1]);
+    }
+  }
+  merge_16(E, O, T);
 }
 
-// Montgomery reduction T * 2^-256 mod m for T < 2^256 * m (fully reduced
-// result).  Eight rows fold the low half: starting from t = T_lo < 2^256, row i
-// adds q_i * m (q_i = t_0 * (-m^-1) mod 2^32) and shifts one word down, so
-// t < 2^256 + 2^32 m stays within nine words and ends at (T_lo + q m) / 2^256
-// <= m.  Adding T_hi < m gives < 2m; one conditional subtraction finishes.
-template <class C>
-__device__ __forceinline__ fe<C> fe_redc(const uint32_t (&T)[16]) {
-  uint32_t t0 = T[0], t1 = T[1], t2 = T[2], t3 = T[3], t4 = T[4], t5 = T[5], t6 = T[6], t7 = T[7];
-  uint32_t t8 = 0;
+// T[0..15] = a^2 for any 256-bit a: the 28 cross products once, in two
+// accumulators by the parity of their position, doubled, and the eight squares
+// as one chain of aligned pairs (36 pairs instead of 64).  A chain marked
+// _top is the first to reach its last pair (beside a carry).
+__device__ __forceinline__ void fe_sqr_wide(const uint32_t (&a)[8], uint32_t (&T)[16]) {
+  uint32_t E[16], O[16];
+  E[0] = E[1] = 0;
+  mul_pair(O, a[1], a[0]);
+  mul_pair(O + 2, a[3], a[0]);
+  mul_pair(O + 4, a[5], a[0]);
+  mul_pair(O + 6, a[7], a[0]);
+  mul_pair(E + 2, a[2], a[0]);
+  mul_pair(E + 4, a[4], a[0]);
+  mul_pair(E + 6, a[6], a[0]);
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint32_t m = t0 * C::INV;
-    ZK_RED_EVEN(m);
-    ZK_RED_ODD(m);
-    t0 = t1; t1 = t2; t2 = t3; t3 = t4; t4 = t5; t5 = t6; t6 = t7; t7 = t8; t8 = 0;
+  for (int i = 8; i < 16; i++) E[i] = O[i] = 0;
+  mac3(O + 2, O[8], a[2], a[4], a[6], a[1]);
+  mac3_top(E + 4, a[3], a[5], a[7], a[1]);
+  mac3_top(O + 4, a[3], a[5], a[7], a[2]);
+  mac2(E + 6, E[10], a[4], a[6], a[2]);
+  mac2(O + 6, O[10], a[4], a[6], a[3]);
+  mac2_top(E + 8, a[5], a[7], a[3]);
+  mac2_top(O + 8, a[5], a[7], a[4]);
+  mac1(E + 10, E[12], a[6], a[4]);
+  mac1(O + 10, O[12], a[6], a[5]);
+  mac1_top(E + 12, a[7], a[5]);
+  mac1_top(O + 12, a[7], a[6]);
+  merge_16(E, O, T);
+#pragma unroll
+  for (int i = 15; i > 0; i--) T[i] = __funnelshift_l(T[i - 1], T[i], 1);
+  T[0] = 0;
+  asm("mad.lo.cc.u32  %0, %16, %16, %0;\n\t"
+      "madc.hi.cc.u32 %1, %16, %16, %1;\n\t"
+      "madc.lo.cc.u32 %2, %17, %17, %2;\n\t"
+      "madc.hi.cc.u32 %3, %17, %17, %3;\n\t"
+      "madc.lo.cc.u32 %4, %18, %18, %4;\n\t"
+      "madc.hi.cc.u32 %5, %18, %18, %5;\n\t"
+      "madc.lo.cc.u32 %6, %19, %19, %6;\n\t"
+      "madc.hi.cc.u32 %7, %19, %19, %7;\n\t"
+      "madc.lo.cc.u32 %8, %20, %20, %8;\n\t"
+      "madc.hi.cc.u32 %9, %20, %20, %9;\n\t"
+      "madc.lo.cc.u32 %10, %21, %21, %10;\n\t"
+      "madc.hi.cc.u32 %11, %21, %21, %11;\n\t"
+      "madc.lo.cc.u32 %12, %22, %22, %12;\n\t"
+      "madc.hi.cc.u32 %13, %22, %22, %13;\n\t"
+      "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
+      "madc.hi.u32    %15, %23, %23, %15;"
+      : "+r"(T[0]), "+r"(T[1]), "+r"(T[2]), "+r"(T[3]), "+r"(T[4]), "+r"(T[5]), "+r"(T[6]),
+        "+r"(T[7]), "+r"(T[8]), "+r"(T[9]), "+r"(T[10]), "+r"(T[11]), "+r"(T[12]), "+r"(T[13]),
+        "+r"(T[14]), "+r"(T[15])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
+}
+
+// One row of the reduction.  s: accumulator whose pairs start at the row's
+// position, o: the other one, whose pairs start a word later.  The row's word
+// is s[0] + o_low (the high half of o's previous pair); its carry enters the
+// odd-limb chain.  q m clears the word, so the row leaves s[0] = 0 and the
+// next row's word is s[1] + o[0].
+template <class C>
+__device__ __forceinline__ void redc_row(uint32_t* s, uint32_t* o, uint32_t o_low) {
+  uint32_t q;
+  asm("add.cc.u32     %0, %0, %18;\n\t"
+      "mul.lo.u32     %17, %0, %19;\n\t"
+      "madc.lo.cc.u32 %9, %17, %21, %9;\n\t"
+      "madc.hi.cc.u32 %10, %17, %21, %10;\n\t"
+      "madc.lo.cc.u32 %11, %17, %23, %11;\n\t"
+      "madc.hi.cc.u32 %12, %17, %23, %12;\n\t"
+      "madc.lo.cc.u32 %13, %17, %25, %13;\n\t"
+      "madc.hi.cc.u32 %14, %17, %25, %14;\n\t"
+      "madc.lo.cc.u32 %15, %17, %27, %15;\n\t"
+      "madc.hi.u32    %16, %17, %27, %16;\n\t"
+      "mad.lo.cc.u32  %0, %17, %20, %0;\n\t"
+      "madc.hi.cc.u32 %1, %17, %20, %1;\n\t"
+      "madc.lo.cc.u32 %2, %17, %22, %2;\n\t"
+      "madc.hi.cc.u32 %3, %17, %22, %3;\n\t"
+      "madc.lo.cc.u32 %4, %17, %24, %4;\n\t"
+      "madc.hi.cc.u32 %5, %17, %24, %5;\n\t"
+      "madc.lo.cc.u32 %6, %17, %26, %6;\n\t"
+      "madc.hi.cc.u32 %7, %17, %26, %7;\n\t"
+      "addc.u32       %8, %8, 0;"
+      : "+r"(s[0]), "+r"(s[1]), "+r"(s[2]), "+r"(s[3]), "+r"(s[4]), "+r"(s[5]), "+r"(s[6]),
+        "+r"(s[7]), "+r"(s[8]), "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]),
+        "+r"(o[5]), "+r"(o[6]), "+r"(o[7]), "=&r"(q)
+      : "r"(o_low), "n"(C::INV), "n"(C::P0), "n"(C::P1), "n"(C::P2), "n"(C::P3), "n"(C::P4),
+        "n"(C::P5), "n"(C::P6), "n"(C::P7));
+}
+
+// Montgomery reduction T * 2^-256 mod m, below m + T / 2^256 (below 2m for
+// T < 2^256 m; the result always fits 256 bits when T_hi <= 2^256 - m).
+// Eight rows fold the low half: row i adds q_i m 2^(32 i) with q_i = t_i
+// (-m^-1) mod 2^32, where t_i is the sum's word i, so after it
+// T_lo + sum q_j m 2^(32 j) is a multiple of 2^(32 (i + 1)) below
+// 2^(32 (i + 9)): the odd-limb chain's last pair (m's top word is below 2^30)
+// carries nothing out, and the even-limb chain's carry is the first thing in
+// its word.  The two accumulators, with pairs at even (A) and odd (B)
+// positions, trade places in every row.  T_hi is added at the end.
+template <class C>
+__device__ __forceinline__ fe<C> fe_redc_lazy(const uint32_t (&T)[16]) {
+  uint32_t A[16], B[16];  // word k of B is position k; B[0] is unused
+#pragma unroll
+  for (int i = 0; i < 8; i++) A[i] = T[i];
+#pragma unroll
+  for (int i = 8; i < 16; i++) A[i] = 0;
+#pragma unroll
+  for (int i = 0; i < 16; i++) B[i] = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    redc_row<C>(A + i, B + i + 1, B[i]);
+    redc_row<C>(B + i + 1, A + i + 2, A[i + 1]);
   }
   fe<C> r;
   asm("add.cc.u32  %0, %8, %16;\n\t"
@@ -468,8 +461,27 @@ __device__ __forceinline__ fe<C> fe_redc(const uint32_t (&T)[16]) {
       "addc.u32    %7, %15, %23;"
       : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
         "=r"(r.v[6]), "=r"(r.v[7])
-      : "r"(t0), "r"(t1), "r"(t2), "r"(t3), "r"(t4), "r"(t5), "r"(t6), "r"(t7), "r"(T[8]),
-        "r"(T[9]), "r"(T[10]), "r"(T[11]), "r"(T[12]), "r"(T[13]), "r"(T[14]), "r"(T[15]));
+      : "r"(A[8]), "r"(A[9]), "r"(A[10]), "r"(A[11]), "r"(A[12]), "r"(A[13]), "r"(A[14]),
+        "r"(A[15]), "r"(B[8]), "r"(B[9]), "r"(B[10]), "r"(B[11]), "r"(B[12]), "r"(B[13]),
+        "r"(B[14]), "r"(B[15]));
+  asm("add.cc.u32  %0, %0, %8;\n\t"
+      "addc.cc.u32 %1, %1, %9;\n\t"
+      "addc.cc.u32 %2, %2, %10;\n\t"
+      "addc.cc.u32 %3, %3, %11;\n\t"
+      "addc.cc.u32 %4, %4, %12;\n\t"
+      "addc.cc.u32 %5, %5, %13;\n\t"
+      "addc.cc.u32 %6, %6, %14;\n\t"
+      "addc.u32    %7, %7, %15;"
+      : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]),
+        "+r"(r.v[6]), "+r"(r.v[7])
+      : "r"(T[8]), "r"(T[9]), "r"(T[10]), "r"(T[11]), "r"(T[12]), "r"(T[13]), "r"(T[14]),
+        "r"(T[15]));
+  return r;
+}
+// fully reduced, for T < 2^256 m
+template <class C>
+__device__ __forceinline__ fe<C> fe_redc(const uint32_t (&T)[16]) {
+  fe<C> r = fe_redc_lazy<C>(T);
   fe_reduce_once<C>(r.v);
   return r;
 }
@@ -497,7 +509,7 @@ __device__ __forceinline__ fe<C> operator*(const fe<C>& a, const fe<C>& b) {
   return fe_mul_call<C>(a, b);
 }
 
-// Out-of-line square (aL^2 + 2 aL aH 2^128 + aH^2 2^256, then REDC).
+// Out-of-line square.
 template <class C>
 __device__ __noinline__ fe<C> fe_sqr_call(fe<C> a) {
   uint32_t T[16];
