@@ -1,0 +1,85 @@
+"""The group operations by lane groups (curve_quad.cuh) at the sizes where the
+bucket reductions, block trees and later accumulation levels can go wrong, on
+both groups, bit-exact against the CPU oracle: one bucket chunk per window,
+several passes, partial segments, repeated points (doublings inside the trees),
+cancelling pairs and buckets left empty."""
+import numpy as np
+import pytest
+
+from _oracle import R, arr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def api():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from zyklop_b200 import api as A
+    return A
+
+
+@pytest.fixture(scope="module")
+def points(api):
+    rng = np.random.default_rng(77)
+    ks = [int.from_bytes(rng.bytes(32), "little") % R for _ in range(60)]
+    return {g: api.mul_generator(g, arr(ks)) for g in (1, 2)}
+
+
+def inputs(points, group, n, kind, rng):
+    xs, ys = points[group]
+    idx = np.arange(n) % len(xs)
+    if kind == "one_point":
+        idx[:] = 3
+    k = [int.from_bytes(rng.bytes(32), "little") % R for _ in range(n)]
+    if kind == "same_scalar":
+        k = [k[0]] * n
+    elif kind == "cancel":  # k P + (r - k) P in pairs, one pair left over if n is odd
+        idx = (np.arange(n) // 2) % len(xs)
+        k = [k[i] if i % 2 == 0 else (R - k[i - 1]) % R for i in range(n)]
+    elif kind == "sparse":
+        k = [v & 0xff if i % 3 else 0 for i, v in enumerate(k)]
+    return xs[idx].copy(), ys[idx].copy(), arr(k)
+
+
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("c,chunk", [(4, 2), (4, 16), (7, 2), (9, 2), (11, 4), (13, 2)])
+def test_bucket_reduction_shapes(api, oracle, points, group, c, chunk):
+    rng = np.random.default_rng(c * 100 + chunk)
+    n = 400 if group == 1 else 150
+    px, py, sc = inputs(points, group, n, "uniform", rng)
+    exp, einf = (oracle.msm_g1 if group == 1 else oracle.msm_g2)(px, py, sc)
+    try:
+        api.msm_set_config(group, c=c, k0=4, k1=2, chunk=chunk)
+        out, inf = (api.msm_g1 if group == 1 else api.msm_g2)(px, py, sc)
+    finally:
+        api.msm_set_config(group)
+    assert inf == bool(einf) and np.array_equal(out, exp)
+
+
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("n", [1, 2, 33, 257])
+@pytest.mark.parametrize("kind", ["one_point", "same_scalar", "cancel", "sparse"])
+def test_equal_points_and_cancellation(api, oracle, points, group, n, kind):
+    rng = np.random.default_rng(n)
+    px, py, sc = inputs(points, group, n, kind, rng)
+    exp, einf = (oracle.msm_g1 if group == 1 else oracle.msm_g2)(px, py, sc)
+    for k0, k1 in ((2, 2), (16, 16)):
+        try:
+            api.msm_set_config(group, c=5, k0=k0, k1=k1, chunk=2)
+            out, inf = (api.msm_g1 if group == 1 else api.msm_g2)(px, py, sc)
+        finally:
+            api.msm_set_config(group)
+        assert inf == bool(einf) and np.array_equal(out, exp)
+
+
+@pytest.mark.parametrize("group,c", [(1, 8), (1, 13), (2, 8), (2, 12)])
+def test_fixed_base_reduction(api, oracle, points, group, c):
+    rng = np.random.default_rng(c)
+    px, py, sc = inputs(points, group, 120, "uniform", rng)
+    exp, _ = (oracle.msm_g1 if group == 1 else oracle.msm_g2)(px, py, sc)
+    t = api.MsmTable(group, px, py, c=c)
+    out, inf = t.run(sc)
+    t.close()
+    assert not inf and np.array_equal(out, exp)

@@ -590,6 +590,32 @@ __device__ __forceinline__ void sub_16(uint32_t (&x)[16], const uint32_t (&y)[16
         "r"(y[15]));
 }
 
+// x[0..15] += y[0..15]; the caller guarantees x + y < 2^512.
+__device__ __forceinline__ void add_16(uint32_t (&x)[16], const uint32_t (&y)[16]) {
+  asm("add.cc.u32  %0, %0, %16;\n\t"
+      "addc.cc.u32 %1, %1, %17;\n\t"
+      "addc.cc.u32 %2, %2, %18;\n\t"
+      "addc.cc.u32 %3, %3, %19;\n\t"
+      "addc.cc.u32 %4, %4, %20;\n\t"
+      "addc.cc.u32 %5, %5, %21;\n\t"
+      "addc.cc.u32 %6, %6, %22;\n\t"
+      "addc.cc.u32 %7, %7, %23;\n\t"
+      "addc.cc.u32 %8, %8, %24;\n\t"
+      "addc.cc.u32 %9, %9, %25;\n\t"
+      "addc.cc.u32 %10, %10, %26;\n\t"
+      "addc.cc.u32 %11, %11, %27;\n\t"
+      "addc.cc.u32 %12, %12, %28;\n\t"
+      "addc.cc.u32 %13, %13, %29;\n\t"
+      "addc.cc.u32 %14, %14, %30;\n\t"
+      "addc.u32    %15, %15, %31;"
+      : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]),
+        "+r"(x[7]), "+r"(x[8]), "+r"(x[9]), "+r"(x[10]), "+r"(x[11]), "+r"(x[12]), "+r"(x[13]),
+        "+r"(x[14]), "+r"(x[15])
+      : "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]),
+        "r"(y[8]), "r"(y[9]), "r"(y[10]), "r"(y[11]), "r"(y[12]), "r"(y[13]), "r"(y[14]),
+        "r"(y[15]));
+}
+
 // y = x + p^2 (p the base-field modulus; every caller's x + p^2 < 2^512).
 __device__ __forceinline__ void add_16_psq(const uint32_t (&x)[16], uint32_t (&y)[16]) {
   asm("add.cc.u32  %0, %16, 0x275d69b1;\n\t"

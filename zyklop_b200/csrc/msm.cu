@@ -7,7 +7,7 @@
 #include <cstring>
 #include <vector>
 
-#include "curve.cuh"
+#include "curve_quad.cuh"
 #include "host_field.hpp"
 #include "msm.hpp"
 #include "profile.hpp"
@@ -18,7 +18,14 @@ namespace {
 
 constexpr uint32_t kInvalid = 0xffffffffu;
 constexpr uint32_t kNeg = 0x80000000u;
-constexpr int kRedT = 128;  // pairs per block in the bucket-reduction block passes
+// pairs per block in the bucket-reduction block passes
+template <class F>
+constexpr int red_pairs() { return sizeof(F) == 64 ? 64 : 128; }
+constexpr int red_pairs(bool g2) { return g2 ? 64 : 128; }
+// nodes per block (a quad each) of the later levels of the segmented reduction
+constexpr int lvl_nodes(bool g2) { return g2 ? 64 : 128; }
+template <class F>
+constexpr int lvl_nodes() { return lvl_nodes(sizeof(F) == 64); }
 
 // ------------------------------------------------------------------ shape
 struct Shape {
@@ -111,7 +118,7 @@ Layout<F> carve(void* base, const Shape& s) {
     L.pkey[i] = cv.take<uint32_t>(pmax[i]);
     L.ppt[i] = cv.take<xyzz<F>>(pmax[i]);
   }
-  const size_t j2 = (s.J + kRedT - 1) / kRedT;
+  const size_t j2 = (s.J + red_pairs<F>() - 1) / red_pairs<F>();
   L.rrun[0] = cv.take<xyzz<F>>((size_t)s.Wk * s.J);
   L.racc[0] = cv.take<xyzz<F>>((size_t)s.Wk * s.J);
   L.rrun[1] = cv.take<xyzz<F>>((size_t)s.Wk * j2);
@@ -263,34 +270,41 @@ struct __align__(16) SegNode {
 template <class F>
 constexpr int seg_threads() { return sizeof(F) == 32 ? 128 : 64; }
 
+// a = a ++ b by the lanes of a quad (every lane of the warp calls it;
+// `on`: whether this quad has a merge to do).
 template <class F>
-__device__ __forceinline__ void seg_merge(SegNode<F>& a, const SegNode<F>& b, xyzz<F>* buckets) {
-  if (b.fk == kInvalid) return;
-  if (a.fk == kInvalid) {
-    a = b;
-    return;
-  }
-  if (a.lk == b.fk) {
-    const xyzz<F> j = xyzz_add(a.single ? a.f : a.l, b.f);
-    if (a.single && b.single) {
-      a.f = j;
-    } else if (a.single) {
-      a.f = j;
-      a.l = b.l;
-      a.single = 0;
-    } else if (b.single) {
-      a.l = j;
+__device__ __forceinline__ void seg_merge(SegNode<F>& a, const SegNode<F>& b, bool on,
+                                          xyzz<F>* buckets) {
+  const uint32_t afk = a.fk, alk = a.lk, bfk = b.fk, blk = b.lk;
+  const bool as = a.single, bs = b.single;
+  const bool join = on && afk != kInvalid && bfk != kInvalid && alk == bfk;
+  const lane_t<F> al = quad_ld(as ? &a.f : &a.l), bf = quad_ld(&b.f);
+  lane_t<F> sum = bf;
+  if (__any_sync(0xffffffffu, join)) sum = quad_add(al, bf);
+  __syncwarp();
+  if (!on || bfk == kInvalid) return;
+  if (afk == kInvalid) {
+    quad_st(&a.f, bf);
+    quad_st(&a.l, quad_ld(&b.l));
+  } else if (join) {
+    if (as) {
+      quad_st(&a.f, sum);
+      if (!bs) quad_st(&a.l, quad_ld(&b.l));
+    } else if (bs) {
+      quad_st(&a.l, sum);
     } else {
-      st_pod(&buckets[a.lk], j);
-      a.l = b.l;
+      quad_st(&buckets[alk], sum);
+      quad_st(&a.l, quad_ld(&b.l));
     }
-    a.lk = b.lk;
   } else {
-    if (!a.single) st_pod(&buckets[a.lk], a.l);
-    if (!b.single) st_pod(&buckets[b.fk], b.f);
-    a.l = b.single ? b.f : b.l;
-    a.lk = b.lk;
-    a.single = 0;
+    if (!as) quad_st(&buckets[alk], al);
+    if (!bs) quad_st(&buckets[bfk], bf);
+    quad_st(&a.l, quad_ld(bs ? &b.f : &b.l));
+  }
+  if (quad_lane<F>() == 0) {
+    if (afk == kInvalid) a.fk = bfk;
+    a.lk = blk;
+    a.single = afk == kInvalid ? bs : (join && as && bs);
   }
 }
 
@@ -313,18 +327,25 @@ __device__ __forceinline__ void seg_close(SegNode<F>& nd, const xyzz<F>& acc, ui
   }
 }
 
-// Block tree over the per-thread nodes, then emit the block's boundary
-// segments: complete ones go to their buckets, the others become partial
-// records 2*block and 2*block+1 for the next level.
-template <class F>
+// Block tree over N nodes, then emit the block's boundary segments: complete
+// ones go to their buckets, the others become partial records 2*block and
+// 2*block+1 for the next level.  A merge is a quad's; the quads of a level are
+// contiguous, so a level's merges occupy as few warps as hold them.
+template <class F, int N>
 __device__ __forceinline__ void seg_block_finish(SegNode<F>* sm, uint32_t key_before,
                                                  uint32_t key_after, xyzz<F>* buckets,
                                                  uint32_t* okey, xyzz<F>* opt, size_t b) {
-  constexpr int T = seg_threads<F>();
+  constexpr int Q = quad_lanes<F>();
   const int t = threadIdx.x;
   __syncthreads();
-  for (int s = 1; s < T; s <<= 1) {
-    if ((t & (2 * s - 1)) == 0) seg_merge(sm[t], sm[t + s], buckets);
+  for (int s = 1; s < N; s <<= 1) {
+    const int merges = N / (2 * s);
+    for (int m0 = (t & ~31) / Q; m0 < merges; m0 += blockDim.x / Q) {  // warp-uniform
+      const int m = m0 + (t & 31) / Q;
+      const bool on = m < merges;
+      const int i = on ? 2 * s * m : 0;
+      seg_merge(sm[i], sm[i + s], on, buckets);
+    }
     __syncthreads();
   }
   if (t != 0) return;
@@ -424,7 +445,7 @@ __device__ __forceinline__ void accum0_tile(size_t b, SegNode<F>* sm,
     }
     seg_close(nd, acc, cur, buckets);
   }
-  seg_block_finish(sm, key_before, key_after, buckets, okey, opt, b);
+  seg_block_finish<F, T>(sm, key_before, key_after, buckets, okey, opt, b);
 }
 
 // One tile per block.  The G1 form takes 148 registers (three blocks per
@@ -465,39 +486,65 @@ __global__ void __launch_bounds__(seg_threads<F>()) k_msm_accum0_queue(
 }
 
 // Levels >= 1: records are (bucket key, XYZZ partial sum); kInvalid keys
-// carry nothing and only ever separate different keys.
+// carry nothing and only ever separate different keys.  A quad per node: these
+// levels are short lists, bound by the depth of their dependent additions.
 template <class F>
-__global__ void __launch_bounds__(seg_threads<F>()) k_msm_accumN(
+__global__ void __launch_bounds__(lvl_nodes<F>() * quad_lanes<F>()) k_msm_accumN(
     const uint32_t* __restrict__ ikey, const xyzz<F>* __restrict__ ipt, size_t m, int K,
     xyzz<F>* __restrict__ buckets, uint32_t* __restrict__ okey, xyzz<F>* __restrict__ opt) {
-  constexpr int T = seg_threads<F>();
-  __shared__ SegNode<F> sm[T];
-  SegNode<F>& nd = sm[threadIdx.x];
-  nd.fk = nd.lk = kInvalid;
-  nd.single = 1;
-  const size_t bstart = (size_t)blockIdx.x * T * K;
+  constexpr int T = lvl_nodes<F>();
+  extern __shared__ __align__(16) unsigned char smem[];
+  SegNode<F>* sm = reinterpret_cast<SegNode<F>*>(smem);
+  const int node = threadIdx.x / quad_lanes<F>();
+  SegNode<F>& nd = sm[node];
+  const size_t bstart = min((size_t)blockIdx.x * T * K, m);
   const size_t bend = min(bstart + (size_t)T * K, m);
-  uint32_t key_before = kInvalid, key_after = kInvalid;
-  if (bstart < m) {
-    key_before = bstart ? ikey[bstart - 1] : kInvalid;
-    key_after = bend < m ? ikey[bend] : kInvalid;
-    const size_t s = bstart + (size_t)threadIdx.x * K;
-    const size_t e = min(s + K, bend);
-    xyzz<F> acc = xyzz_inf<F>();
-    uint32_t cur = kInvalid;
-    for (size_t p = s; p < e; p++) {
-      const uint32_t key = ikey[p];
-      if (key == kInvalid) continue;
-      if (key != cur) {
-        seg_close(nd, acc, cur, buckets);
-        cur = key;
-        acc = xyzz_inf<F>();
-      }
-      acc = xyzz_add(acc, ld_pod(ipt + p));
+  const uint32_t key_before = bstart && bstart < m ? ikey[bstart - 1] : kInvalid;
+  const uint32_t key_after = bend < m ? ikey[bend] : kInvalid;
+  const size_t s = bstart + (size_t)node * K;
+  // the node's segments so far (registers of all four lanes; `acc` and the
+  // closed segments one coordinate per lane)
+  uint32_t fk = kInvalid, lk = kInvalid, cur = kInvalid;
+  bool single = true;
+  lane_t<F> acc = quad_inf<F>(), f = acc, l = acc;
+  auto close = [&] {
+    if (cur == kInvalid) return;
+    if (fk == kInvalid) {
+      fk = lk = cur;
+      f = acc;
+    } else {
+      if (!single) quad_st(&buckets[lk], l);
+      lk = cur;
+      l = acc;
+      single = false;
     }
-    seg_close(nd, acc, cur, buckets);
+  };
+  for (int i = 0; i < K; i++) {
+    const size_t p = s + i;
+    const uint32_t key = p < bend ? ikey[p] : kInvalid;
+    const bool on = key != kInvalid;
+    if (!__any_sync(0xffffffffu, on)) continue;
+    const lane_t<F> v = on ? quad_ld(ipt + p) : quad_inf<F>();
+    const bool same = on && key == cur;
+    lane_t<F> sum = v;
+    if (__any_sync(0xffffffffu, same)) sum = quad_add(acc, v);
+    if (on && !same) {
+      close();
+      cur = key;
+      acc = v;
+    } else if (on) {
+      acc = sum;
+    }
   }
-  seg_block_finish(sm, key_before, key_after, buckets, okey, opt, (size_t)blockIdx.x);
+  close();
+  quad_st(&nd.f, f);
+  quad_st(&nd.l, l);
+  if (quad_lane<F>() == 0) {
+    nd.fk = fk;
+    nd.lk = lk;
+    nd.single = single;
+  }
+  seg_block_finish<F, T>(sm, key_before, key_after, buckets, okey, opt, (size_t)blockIdx.x);
 }
 
 // dst[i] += src[i]: the buckets of two MSMs whose results are added, so one
@@ -515,13 +562,15 @@ __global__ void __launch_bounds__(128) k_msm_bucket_add(xyzz<F>* __restrict__ ds
 // Window sums sum_b (b+1) S_b, without per-chunk scalar multiplications and
 // without long serial chains above the first level.
 //
-// Level 1: thread per (window, chunk of L buckets) -> (run, acc) with
+// Additions are quad operations (curve_quad.cuh): these are dependent chains
+// on a device that is far from full.
+// Level 1: quad per (window, chunk of L buckets) -> (run, acc) with
 // run = sum S_b and acc = sum (i+1) S_{lo+i} (running sums from the top).
-// Block passes: block per (window, segment of up to kRedT consecutive pairs,
+// Block passes: block per (window, segment of up to red_pairs consecutive pairs,
 // each covering 2^log_span buckets) -> run' = sum run_i and
 // acc' = sum acc_i + 2^log_span * sum_i i run_i.  In the block,
 // sum_i i run_i = sum_{i>=1} S_i with S_i = sum_{k>=i} run_k: a shared-memory
-// suffix scan (log2 kRedT steps) and a tree reduction, so the depth is
+// suffix scan (log2 of the pairs, in steps) and a tree reduction, so the depth is
 // logarithmic.  The final pass (one segment per window) stops before the
 // doublings and leaves U = sum_i i run_i and A = sum_i acc_i; the host forms
 // the window sum A + 2^log_span U, where a serial doubling chain is cheap.
@@ -530,56 +579,62 @@ __global__ void __launch_bounds__(128) k_msm_reduce_l1(const xyzz<F>* __restrict
                                                        int W, uint32_t B, uint32_t L, uint32_t J,
                                                        xyzz<F>* __restrict__ run_out,
                                                        xyzz<F>* __restrict__ acc_out) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)W * J) return;
-  const int w = (int)(t / J);
+  const size_t t = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / quad_lanes<F>();
+  const bool on = t < (size_t)W * J;
+  const int w = on ? (int)(t / J) : 0;
   const uint32_t j = (uint32_t)(t % J);
   const int nbits = 256 - w * c;
   const uint32_t Bw = nbits >= c ? B : (nbits <= 0 ? 1u : (1u << nbits));
-  const uint32_t lo = j * L;
-  xyzz<F> run = xyzz_inf<F>(), acc = xyzz_inf<F>();
-  if (lo < Bw) {
-    const uint32_t hi = min(lo + L, Bw);
-    const xyzz<F>* bw = buckets + (size_t)w * B;
-    for (uint32_t b = hi; b-- > lo;) {
-      run = xyzz_add(run, ld_pod(bw + b));
-      acc = xyzz_add(acc, run);
-    }
+  const uint32_t lo = on ? min(j * L, Bw) : 0, hi = on ? min(lo + L, Bw) : 0;
+  const xyzz<F>* bw = buckets + (size_t)w * B;
+  lane_t<F> run = quad_inf<F>(), acc = run;
+  for (uint32_t i = L; i-- > 0;) {
+    const bool has = lo + i < hi;
+    if (!__any_sync(0xffffffffu, has)) continue;
+    run = quad_add(run, has ? quad_ld(bw + lo + i) : quad_inf<F>());
+    acc = quad_add(acc, run);
   }
-  st_pod(&run_out[t], run);
-  st_pod(&acc_out[t], acc);
+  if (!on) return;
+  quad_st(&run_out[t], run);
+  quad_st(&acc_out[t], acc);
 }
 
-// block tree sum over the first `width` threads' values (a power of two;
-// result valid in thread 0)
+// tree sum over the first `width` quads' values (a power of two; result valid
+// in quad 0)
 template <class F>
-__device__ __forceinline__ xyzz<F> block_sum(xyzz<F> v, xyzz<F>* sm, int width) {
-  const int i = threadIdx.x;
-  sm[i] = v;
+__device__ __forceinline__ lane_t<F> block_sum(lane_t<F> v, xyzz<F>* sm, int width) {
+  constexpr int Q = quad_lanes<F>();
+  const int i = threadIdx.x / Q, i0 = (threadIdx.x & ~31) / Q;
+  quad_st(&sm[i], v);
   __syncthreads();
   for (int s = width / 2; s > 0; s >>= 1) {
-    if (i < s) sm[i] = xyzz_add(sm[i], sm[i + s]);
+    if (i0 < s) {  // warp-uniform
+      v = quad_add(v, quad_ld(&sm[min(i + s, red_pairs<F>() - 1)]));
+      __syncwarp();
+      if (i < s) quad_st(&sm[i], v);
+    }
     __syncthreads();
   }
-  const xyzz<F> r = sm[0];
+  v = quad_ld(&sm[0]);
   __syncthreads();
-  return r;
+  return v;
 }
 
 // grid (segments, windows); out_u / out_a receive U and A of final passes.
 // Depth: the scan and the trees run over the segment's width (the power of
 // two covering its pairs), not the whole block.  When the doublings are few
 // (always between passes, and in a final pass when log_span + 1 is below the
-// tree depth) each thread folds 2^log_span S_i into its acc_i and one tree
+// tree depth) each quad folds 2^log_span S_i into its acc_i and one tree
 // sums the result, instead of two trees and a serial doubling tail; a final
 // pass then leaves U = infinity and the whole sum in A.
 template <class F>
-__global__ void __launch_bounds__(kRedT) k_msm_reduce_blk(
+__global__ void __launch_bounds__(red_pairs<F>() * quad_lanes<F>()) k_msm_reduce_blk(
     const xyzz<F>* __restrict__ run_in, const xyzz<F>* __restrict__ acc_in, uint32_t Jin,
     int log_span, uint32_t Jout, xyzz<F>* __restrict__ run_out, xyzz<F>* __restrict__ acc_out,
     xyzz<F>* __restrict__ out_u, xyzz<F>* __restrict__ out_a) {
+  constexpr int kRedT = red_pairs<F>(), Q = quad_lanes<F>();
   __shared__ xyzz<F> sm[kRedT];
-  const int w = blockIdx.y, i = threadIdx.x;
+  const int w = blockIdx.y, i = threadIdx.x / Q, i0 = (threadIdx.x & ~31) / Q;
   const uint32_t idx = blockIdx.x * kRedT + i;
   const size_t base = (size_t)w * Jin;
   const uint32_t len = min((uint32_t)kRedT, Jin - blockIdx.x * kRedT);
@@ -588,41 +643,48 @@ __global__ void __launch_bounds__(kRedT) k_msm_reduce_blk(
     width <<= 1;
     depth++;
   }
-  xyzz<F> r = idx < Jin ? ld_pod(run_in + base + idx) : xyzz_inf<F>();
+  const lane_t<F> zero = quad_inf<F>();
+  lane_t<F> r = idx < Jin ? quad_ld(run_in + base + idx) : zero;
   // inclusive suffix scan: r = S_i = sum_{k >= i} run_k within the segment
-  sm[i] = r;
+  quad_st(&sm[i], r);
   __syncthreads();
   for (int off = 1; off < width; off <<= 1) {
-    const xyzz<F> o = i + off < kRedT ? sm[i + off] : xyzz_inf<F>();
+    const lane_t<F> o = i + off < kRedT ? quad_ld(&sm[i + off]) : zero;
     __syncthreads();
-    r = xyzz_add(r, o);
-    sm[i] = r;
+    if (i0 < width) {  // warp-uniform
+      r = quad_add(r, o);
+      quad_st(&sm[i], r);
+    }
     __syncthreads();
   }
-  const xyzz<F> total = sm[0];  // S_0 = sum of the segment's runs
+  const lane_t<F> total = quad_ld(&sm[0]);  // S_0 = sum of the segment's runs
   __syncthreads();
-  const xyzz<F> acc = idx < Jin ? ld_pod(acc_in + base + idx) : xyzz_inf<F>();
+  const lane_t<F> acc = idx < Jin ? quad_ld(acc_in + base + idx) : zero;
   const size_t o = (size_t)w * Jout + blockIdx.x;
+  if (i == 0) r = zero;
   if (Jout > 1 || log_span + 1 < depth) {
-    xyzz<F> t = i >= 1 ? r : xyzz_inf<F>();
-    for (int d = 0; d < log_span; d++) t = xyzz_dbl(t);
-    const xyzz<F> s = block_sum<F>(xyzz_add(t, acc), sm, width);
+    lane_t<F> t = zero;
+    if (i0 < width) {
+      for (int d = 0; d < log_span; d++) r = quad_dbl(r);
+      t = quad_add(r, acc);
+    }
+    const lane_t<F> s = block_sum<F>(t, sm, width);
     if (i != 0) return;
     if (Jout == 1) {
-      st_pod(&out_u[w], xyzz_inf<F>());
-      st_pod(&out_a[w], s);
+      quad_st(&out_u[w], zero);
+      quad_st(&out_a[w], s);
     } else {
-      st_pod(&run_out[o], total);
-      st_pod(&acc_out[o], s);
+      quad_st(&run_out[o], total);
+      quad_st(&acc_out[o], s);
     }
     return;
   }
   // final pass with many doublings: U and A separately, the host doubles U
-  const xyzz<F> u = block_sum<F>(i >= 1 ? r : xyzz_inf<F>(), sm, width);
-  const xyzz<F> a = block_sum<F>(acc, sm, width);
+  const lane_t<F> u = block_sum<F>(r, sm, width);
+  const lane_t<F> a = block_sum<F>(acc, sm, width);
   if (i != 0) return;
-  st_pod(&out_u[w], u);
-  st_pod(&out_a[w], a);
+  quad_st(&out_u[w], u);
+  quad_st(&out_a[w], a);
 }
 
 // ------------------------------------------------------ fixed-base tables
@@ -759,7 +821,8 @@ MsmResult msm_enqueue(const ScalarSrc& ss, const PointSrc<F>& ps, int inst, size
   for (int l = 1; l < s.levels; l++) {
     const int in = l & 1, out = in ^ 1;
     uint32_t* ok = (l + 1 < s.levels) ? L.pkey[out] : nullptr;
-    k_msm_accumN<F><<<(unsigned)s.lvl_blocks[l], seg_threads<F>(), 0, st>>>(
+    k_msm_accumN<F><<<(unsigned)s.lvl_blocks[l], lvl_nodes<F>() * quad_lanes<F>(),
+                      lvl_nodes<F>() * sizeof(SegNode<F>), st>>>(
         L.pkey[in], L.ppt[in], s.lvl_records[l], s.lvl_k[l], L.buckets, ok, L.ppt[out]);
     ZK_LAUNCHED();
   }
@@ -792,20 +855,21 @@ MsmResult msm_enqueue(const ScalarSrc& ss, const PointSrc<F>& ps, int inst, size
     const uint32_t Lc = (uint32_t)s.chunk;
     while ((1u << log_span) < Lc) log_span++;
     const size_t tot = (size_t)s.Wk * J;
-    k_msm_reduce_l1<F><<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(
+    k_msm_reduce_l1<F><<<(unsigned)((quad_lanes<F>() * tot + 127) / 128), 128, 0, st>>>(
         L.buckets, s.fixed ? 0 : s.c, s.Wk, s.B, Lc, J, L.rrun[0], L.racc[0]);
     ZK_LAUNCHED();
     int cur = 0;
     for (;;) {
+      constexpr int kRedT = red_pairs<F>();
       const uint32_t Jout = (J + kRedT - 1) / kRedT;
-      k_msm_reduce_blk<F><<<dim3(Jout, s.Wk), kRedT, 0, st>>>(
+      k_msm_reduce_blk<F><<<dim3(Jout, s.Wk), kRedT * quad_lanes<F>(), 0, st>>>(
           L.rrun[cur], L.racc[cur], J, log_span, Jout, L.rrun[cur ^ 1], L.racc[cur ^ 1], L.outua,
           L.outua + s.Wk);
       ZK_LAUNCHED();
       if (Jout == 1) break;
       cur ^= 1;
       J = Jout;
-      log_span += 7;  // kRedT = 2^7 pairs per block
+      log_span += g2 ? 6 : 7;  // log2 of the pairs per block
     }
   }
   MsmResult res;
