@@ -528,10 +528,16 @@ __device__ __forceinline__ fe<C> fe_to_mont(const fe<C>& a) {
   const fe<C> r2{{C::R2[0], C::R2[1], C::R2[2], C::R2[3], C::R2[4], C::R2[5], C::R2[6], C::R2[7]}};
   return a * r2;
 }
+// a R^-1: the reduction alone
 template <class C>
 __device__ __forceinline__ fe<C> fe_from_mont(const fe<C>& a) {
-  const fe<C> one{{1, 0, 0, 0, 0, 0, 0, 0}};
-  return a * one;
+  uint32_t T[16];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    T[i] = a.v[i];
+    T[8 + i] = 0;
+  }
+  return fe_redc<C>(T);
 }
 
 // a^e for a small public exponent given as 8 x u32 limbs (square-and-multiply)

@@ -16,8 +16,14 @@
 namespace zk {
 namespace {
 
-constexpr int kTile = 1024;       // elements per pass tile
-constexpr int kPassThreads = 256;
+constexpr int kTile = 512;               // elements per pass tile
+constexpr int kPassThreads = kTile / 4;  // one radix-4 group per thread and stage pair
+constexpr int kPassBlocks = 5;           // resident per SM
+constexpr int kElemThreads = 256;        // elementwise kernels
+
+// 2r
+constexpr uint32_t k2R[8] = {0xe0000002u, 0x87c3eb27u, 0xf372e122u, 0x5067d090u,
+                             0x0302b0bau, 0x70a08b6du, 0xc2634053u, 0x60c89ce5u};
 
 using host::Fr;
 
@@ -46,6 +52,90 @@ __global__ void k_tw_fill(fr_t* __restrict__ out, const fr_t* __restrict__ hi,
   fe_store(out, e, a * b);
 }
 
+// ------------------------------------------------ partly reduced values
+// x - 2r if x >= 2r
+__device__ __forceinline__ void fr_reduce_2r(fr_t& x) {
+  uint32_t s[8], bw;
+  asm("sub.cc.u32  %0, %9, %17;\n\t"
+      "subc.cc.u32 %1, %10, %18;\n\t"
+      "subc.cc.u32 %2, %11, %19;\n\t"
+      "subc.cc.u32 %3, %12, %20;\n\t"
+      "subc.cc.u32 %4, %13, %21;\n\t"
+      "subc.cc.u32 %5, %14, %22;\n\t"
+      "subc.cc.u32 %6, %15, %23;\n\t"
+      "subc.cc.u32 %7, %16, %24;\n\t"
+      "subc.u32    %8, 0, 0;"
+      : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]),
+        "=r"(s[7]), "=r"(bw)
+      : "r"(x.v[0]), "r"(x.v[1]), "r"(x.v[2]), "r"(x.v[3]), "r"(x.v[4]), "r"(x.v[5]),
+        "r"(x.v[6]), "r"(x.v[7]), "n"(k2R[0]), "n"(k2R[1]), "n"(k2R[2]), "n"(k2R[3]),
+        "n"(k2R[4]), "n"(k2R[5]), "n"(k2R[6]), "n"(k2R[7]));
+#pragma unroll
+  for (int q = 0; q < 8; q++) x.v[q] = bw ? x.v[q] : s[q];
+}
+__device__ __forceinline__ fr_t fr_add_raw(const fr_t& a, const fr_t& b) {
+  fr_t r;
+  add_raw(a.v, b.v, r.v);
+  return r;
+}
+// a - b + 2r for a, b < 2r
+__device__ __forceinline__ fr_t fr_sub_2r(const fr_t& a, const fr_t& b) {
+  fr_t r;
+  asm("add.cc.u32  %0, %8, %16;\n\t"
+      "addc.cc.u32 %1, %9, %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
+        "=r"(r.v[6]), "=r"(r.v[7])
+      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),
+        "r"(a.v[7]), "n"(k2R[0]), "n"(k2R[1]), "n"(k2R[2]), "n"(k2R[3]), "n"(k2R[4]),
+        "n"(k2R[5]), "n"(k2R[6]), "n"(k2R[7]));
+  asm("sub.cc.u32  %0, %0, %8;\n\t"
+      "subc.cc.u32 %1, %1, %9;\n\t"
+      "subc.cc.u32 %2, %2, %10;\n\t"
+      "subc.cc.u32 %3, %3, %11;\n\t"
+      "subc.cc.u32 %4, %4, %12;\n\t"
+      "subc.cc.u32 %5, %5, %13;\n\t"
+      "subc.cc.u32 %6, %6, %14;\n\t"
+      "subc.u32    %7, %7, %15;"
+      : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]),
+        "+r"(r.v[6]), "+r"(r.v[7])
+      : "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]),
+        "r"(b.v[7]));
+  return r;
+}
+// x 2^-L mod r, below 2r, for x < 2r and 1 <= L <= 31: adds the multiple
+// m r (m < 2^L) that clears the low L bits and shifts; (2r + 2^L r) / 2^L <= 2r.
+// About 35 instructions against a product's 221.
+__device__ __forceinline__ fr_t fr_div_pow2(const fr_t& x, int L) {
+  const uint32_t r[8] = {FrCfg::P0, FrCfg::P1, FrCfg::P2, FrCfg::P3,
+                         FrCfg::P4, FrCfg::P5, FrCfg::P6, FrCfg::P7};
+  const uint32_t m = (x.v[0] * FrCfg::INV) & ((1u << L) - 1);
+  uint32_t y[9];
+  uint64_t c = 0;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    c += (uint64_t)m * r[i] + x.v[i];
+    y[i] = (uint32_t)c;
+    c >>= 32;
+  }
+  y[8] = (uint32_t)c;
+  fr_t o;
+#pragma unroll
+  for (int i = 0; i < 8; i++) o.v[i] = __funnelshift_r(y[i], y[i + 1], L);
+  return o;
+}
+// a w 2^-256 mod r, below 2r, for any 256-bit a and w < r
+__device__ __forceinline__ fr_t fr_mul_lazy(const fr_t& a, const fr_t& w) {
+  uint32_t T[16];
+  fe_mul_wide(a.v, w.v, T);
+  return fe_redc_lazy<FrCfg>(T);
+}
+
 // arrays transformed by one pass launch (blockIdx.y): the three vectors of
 // up to kMaxHBatch H polynomials of one size
 constexpr int kMaxPassArrays = 3 * kMaxHBatch;
@@ -70,11 +160,6 @@ struct HArgs {
 // (radix 4: a thread loads a quad of elements, runs both stages in registers
 // and stores it back, one shared-memory round trip and one barrier for two
 // stages); the butterflies of global bit 0 have w = 1 and skip the product.
-struct NttSlots {
-  const uint32_t* sm;
-  int tile;
-};
-
 __device__ __forceinline__ fr_t sm_load(const uint32_t* sm, int tile, int slot) {
   fr_t x;
 #pragma unroll
@@ -95,17 +180,29 @@ __device__ __forceinline__ fr_t ntt_twiddle(const fr_t* __restrict__ tw, int tw_
   return fe_ldg<FrCfg>(tw, (imod << (L - 1 - (lo + bit))) << tw_shift);
 }
 
+// Between stages and passes values stay partly reduced (Harvey, "Faster
+// arithmetic for number-theoretic transforms", 2014): below 2r in the DIF
+// passes and below 4r < 2^256 in the DIT passes, so a butterfly does one
+// conditional subtraction of 2r instead of three full reductions.  A product
+// of any 256-bit value by a twiddle w < r leaves fe_redc's last step below
+// r + 4r * r / 2^256 < 2r.  The transform's last writer reduces fully.
+//   DIT: u, v < 4r -> u' = u mod 2r; (u' + v w, u' - v w + 2r) < 4r
+//   DIF: u, v < 2r -> ((u + v) mod 2r, (u - v + 2r) w) < 2r
 template <bool DIT>
 __device__ __forceinline__ void butterfly(fr_t& u, fr_t& v, const fr_t& w, bool trivial) {
   if (DIT) {
-    if (!trivial) v = fe_mul_inline(v, w);
-    const fr_t a = u + v;
-    v = u - v;
+    if (trivial) fr_reduce_2r(v);
+    else v = fr_mul_lazy(v, w);
+    fr_reduce_2r(u);
+    const fr_t a = fr_add_raw(u, v);
+    v = fr_sub_2r(u, v);
     u = a;
   } else {
-    const fr_t a = u + v;
-    v = u - v;
-    if (!trivial) v = fe_mul_inline(v, w);
+    fr_t a = fr_add_raw(u, v);
+    v = fr_sub_2r(u, v);
+    if (trivial) fr_reduce_2r(v);
+    else v = fr_mul_lazy(v, w);
+    fr_reduce_2r(a);
     u = a;
   }
 }
@@ -123,12 +220,24 @@ __device__ __forceinline__ fr_t fr_load(const fr_t* base, size_t idx) {
   return fe_load<FrCfg>(base, idx);
 }
 
+// How the last DIF pass (bits [0, k)) of a transform leaves its results: in
+// place (bit-reversed order, below 2r), or canonical in natural order, the
+// inverse transform's divided by N.  The reordering rides on the pass's own
+// store instead of a pass of its own: a block takes groups that differ in
+// their high bits, which land next to each other.
+enum PassOrder { kKeep, kNatural, kNaturalOverN };
+
+__device__ __forceinline__ size_t rev_bits(size_t x, int bits) {
+  return bits ? (size_t)(__brevll((unsigned long long)x) >> (64 - bits)) : 0;
+}
+
 // One tile of a pass (block `blk` of the launch that runs this pass over
 // the array in -> out).
 template <bool DIT, bool CG>
 __device__ __forceinline__ void pass_tile(const fr_t* in, fr_t* out, size_t blk,
                                           const fr_t* __restrict__ tw, int tw_shift, int L, int lo,
-                                          int k, int log_g, uint32_t* sm) {
+                                          int k, int log_g, uint32_t* sm, int order = kKeep) {
+  const bool full = DIT && lo + k == L;  // the last DIT pass leaves canonical values
   const int tile = 1 << (k + log_g);
   const int G = 1 << log_g;
   const size_t gid0 = blk << log_g;
@@ -142,7 +251,9 @@ __device__ __forceinline__ void pass_tile(const fr_t* in, fr_t* out, size_t blk,
       g = e & (G - 1);
       j = e >> log_g;
     }
-    const size_t gid = gid0 + g;
+    size_t gid = gid0 + g;
+    if (order != kKeep)  // groups whose results are neighbours in natural order
+      gid = (rev_bits(g, log_g) << (L - k - log_g)) | blk;
     const size_t idx = ((gid >> lo) << (lo + k)) | ((size_t)j << lo) | (gid & lomask);
     sm_store(sm, tile, (j << log_g) | g, fr_load<CG>(in, idx));
   }
@@ -208,6 +319,18 @@ __device__ __forceinline__ void pass_tile(const fr_t* in, fr_t* out, size_t blk,
     }
     __syncthreads();
   }
+  if (order != kKeep) {
+    // natural order: position rev(idx), with G neighbours per sub-transform index
+    const size_t base = rev_bits(blk, L - k - log_g) << log_g;
+    for (int e = threadIdx.x; e < tile; e += blockDim.x) {
+      const int g = e & (G - 1), j = e >> log_g;
+      fr_t x = sm_load(sm, tile, e);
+      if (order == kNaturalOverN) x = fr_div_pow2(x, L);
+      fe_reduce_once<FrCfg>(x.v);
+      fe_store(out, (rev_bits(j, k) << (L - k)) | base | g, x);
+    }
+    return;
+  }
   for (int e = threadIdx.x; e < tile; e += blockDim.x) {
     int j, g;
     if (lo == 0) {
@@ -219,27 +342,30 @@ __device__ __forceinline__ void pass_tile(const fr_t* in, fr_t* out, size_t blk,
     }
     const size_t gid = gid0 + g;
     const size_t idx = ((gid >> lo) << (lo + k)) | ((size_t)j << lo) | (gid & lomask);
-    fe_store(out, idx, sm_load(sm, tile, (j << log_g) | g));
+    fr_t x = sm_load(sm, tile, (j << log_g) | g);
+    if (full) {
+      fr_reduce_2r(x);
+      fe_reduce_once<FrCfg>(x.v);
+    }
+    fe_store(out, idx, x);
   }
 }
 
+// Bound by the multiply pipe and, between its barriers, by latency.  Five
+// blocks of 128 threads per SM: the radix-4 stage holds four elements beside a
+// product, 122 registers uncapped; capped at 96 it spills ~80 bytes a thread.
+// Forward 2^24: 4.00 ms, 4.11 at four blocks, 4.14 at six; tiles of 1024
+// elements (blocks of 256 threads, two per SM) 4.43, of 256 elements 4.12
+// (their 32-byte column segments cost memory efficiency there).  The H
+// pipeline at 2^20: 1.49 ms, with 1024-element tiles 1.66.
 template <bool DIT>
-__global__ void __launch_bounds__(kPassThreads) k_ntt_pass(PassArgs args, const fr_t* __restrict__ tw,
-                                                           int tw_shift, int L, int lo, int k,
-                                                           int log_g) {
+__global__ void __launch_bounds__(kPassThreads, kPassBlocks) k_ntt_pass(PassArgs args,
+                                                              const fr_t* __restrict__ tw,
+                                                              int tw_shift, int L, int lo, int k,
+                                                              int log_g, int order) {
   extern __shared__ uint32_t sm[];
   pass_tile<DIT, false>(args.in[blockIdx.y], args.out[blockIdx.y], blockIdx.x, tw, tw_shift, L, lo,
-                        k, log_g, sm);
-}
-
-__global__ void k_bitrev(const fr_t* __restrict__ in, fr_t* __restrict__ out, int L, bool scale,
-                         fr_t factor) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >> L) return;
-  const size_t r = L ? (__brevll((unsigned long long)i) >> (64 - L)) : 0;
-  fr_t x = fe_load<FrCfg>(in, i);
-  if (scale) x = x * factor;
-  fe_store(out, r, x);
+                        k, log_g, sm, order);
 }
 
 // C = A * B elementwise
@@ -255,12 +381,14 @@ __global__ void k_pointwise_mul(const __grid_constant__ HArgs args, size_t n) {
 }
 
 // x[p] *= (1/N) omega_2n^rev(p) for coefficients held in bit-reversed order
-// (the coset shift of src/groth16.cu:914-921 with the INTT scale folded in).
+// (the coset shift of src/groth16.cu:914-921 with the INTT scale folded in),
+// for the three vectors of a polynomial at once: the factor is formed once,
+// and 1/N is an exact shift.  Results stay below 2r for the DIT passes.
 template <bool CG>
-__device__ __forceinline__ void coset_elem(fr_t* a, size_t p, const fr_t* __restrict__ tw,
-                                           int tw_shift, int L, const fr_t& c_even,
-                                           const fr_t& c_odd) {
-  const size_t e = L ? (__brevll((unsigned long long)p) >> (64 - L)) : 0;
+__device__ __forceinline__ void coset_elem(fr_t* const (&v)[3], size_t p,
+                                           const fr_t* __restrict__ tw, int tw_shift, int L,
+                                           const fr_t& w2n) {
+  const size_t e = rev_bits(p, L);
   const size_t f = e >> 1;  // omega_2n^e = omega_2n^(e & 1) * omega_N^f
   const size_t half = L ? (size_t(1) << (L - 1)) : 1;
   fr_t t;
@@ -269,14 +397,19 @@ __device__ __forceinline__ void coset_elem(fr_t* a, size_t p, const fr_t* __rest
   } else {
     t = fe_neg(fe_ldg<FrCfg>(tw, (f - half) << tw_shift));  // omega_N^(N/2) = -1
   }
-  fe_store(a, p, fr_load<CG>(a, p) * t * ((e & 1) ? c_odd : c_even));
+  if (e & 1) t = t * w2n;  // the upper half of the positions
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    fe_store(v[q], p, fr_div_pow2(fr_mul_lazy(fr_load<CG>(v[q], p), t), L));
 }
 
 __global__ void k_coset_scale(PassArgs args, const fr_t* __restrict__ tw, int tw_shift, int L,
-                              fr_t c_even, fr_t c_odd) {
+                              fr_t w2n) {
   const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >> L) return;
-  coset_elem<false>(args.in[blockIdx.y], p, tw, tw_shift, L, c_even, c_odd);
+  const int j = 3 * blockIdx.y;
+  fr_t* const v[3] = {args.in[j], args.in[j + 1], args.in[j + 2]};
+  coset_elem<false>(v, p, tw, tw_shift, L, w2n);
 }
 
 // h = A*B - C, decoded to canonical (src/groth16.cu:935-948, 218-226), per
@@ -323,7 +456,7 @@ int split_passes(int L, int maxbits, int* lo, int* k) {
 }
 
 void run_pass(bool dit, const PassArgs& args, int count, const fr_t* tw, int tw_shift, int L, int lo,
-              int k, cudaStream_t st) {
+              int k, cudaStream_t st, int order = kKeep) {
   const size_t groups = size_t(1) << (L - k);
   int log_g = 0;
   while ((1 << (log_g + 1 + k)) <= kTile && (size_t(1) << (log_g + 1)) <= groups &&
@@ -334,19 +467,24 @@ void run_pass(bool dit, const PassArgs& args, int count, const fr_t* tw, int tw_
   dim3 grid((unsigned)blocks, count);
   ProfScope prof(kProfNttPass, (double)count * (double)(size_t(1) << L), st);
   if (dit)
-    k_ntt_pass<true><<<grid, kPassThreads, smem, st>>>(args, tw, tw_shift, L, lo, k, log_g);
+    k_ntt_pass<true><<<grid, kPassThreads, smem, st>>>(args, tw, tw_shift, L, lo, k, log_g, order);
   else
-    k_ntt_pass<false><<<grid, kPassThreads, smem, st>>>(args, tw, tw_shift, L, lo, k, log_g);
+    k_ntt_pass<false><<<grid, kPassThreads, smem, st>>>(args, tw, tw_shift, L, lo, k, log_g, order);
   ZK_LAUNCHED();
 }
 
-// all DIF passes (high bit ranges first); first pass may be out of place
-void dif(const PassArgs& first, const PassArgs& rest, int count, const fr_t* tw, int tw_shift, int L,
-         int maxbits, cudaStream_t st) {
+// all DIF passes (high bit ranges first); the first pass reads `first`'s
+// input, the others run as `rest`, and the last one writes `last`'s output in the given order
+void dif(const PassArgs& first, const PassArgs& rest, const PassArgs& last, int count,
+         const fr_t* tw, int tw_shift, int L, int maxbits, cudaStream_t st, int order = kKeep) {
   int lo[8], k[8];
   const int np = split_passes(L, maxbits, lo, k);
-  for (int i = np - 1; i >= 0; i--)
-    run_pass(false, i == np - 1 ? first : rest, count, tw, tw_shift, L, lo[i], k[i], st);
+  for (int i = np - 1; i >= 0; i--) {
+    PassArgs a = i == 0 ? last : rest;
+    if (i == np - 1)
+      for (int q = 0; q < count; q++) a.in[q] = first.in[q];
+    run_pass(false, a, count, tw, tw_shift, L, lo[i], k[i], st, i == 0 ? order : kKeep);
+  }
 }
 
 void dit(const PassArgs& args, int count, const fr_t* tw, int tw_shift, int L, int maxbits,
@@ -407,14 +545,13 @@ void ntt_inplace(NttTables& tw, uint64_t* a, int log_n, bool inverse, void* scra
   const fr_t* table = inverse ? tw.inv.as<fr_t>() : tw.fwd.as<fr_t>();
   fr_t* x = reinterpret_cast<fr_t*>(a);
   fr_t* s = reinterpret_cast<fr_t*>(scratch);
-  PassArgs first{{x, nullptr, nullptr}, {s, nullptr, nullptr}};
-  PassArgs rest{{s, nullptr, nullptr}, {s, nullptr, nullptr}};
-  dif(first, rest, 1, table, shift, log_n, tw.pass_bits[log_n], st);
-  const size_t n = size_t(1) << log_n;
-  fr_t factor{};
-  if (inverse) factor = to_dev(Fr::from_u64(n).inv());
-  k_bitrev<<<blocks_for(n), 256, 0, st>>>(s, x, log_n, inverse, factor);
-  ZK_LAUNCHED();
+  // first pass x -> s, the passes between in s, the last s -> x (a transform
+  // of one pass is one block: it has read all of x before it writes)
+  PassArgs first{}, rest{}, last{};
+  first.in[0] = last.out[0] = x;
+  rest.in[0] = rest.out[0] = last.in[0] = s;
+  dif(first, rest, last, 1, table, shift, log_n, tw.pass_bits[log_n], st,
+      inverse ? kNaturalOverN : kNatural);
 }
 
 void hpoly_batch(NttTables& tw, int count, uint64_t* const* aw, uint64_t* const* bw,
@@ -437,11 +574,9 @@ void hpoly_batch(NttTables& tw, int count, uint64_t* const* aw, uint64_t* const*
   }
   k_pointwise_mul<<<dim3(blocks_for(n), count), 256, 0, st>>>(ha, n);
   ZK_LAUNCHED();
-  dif(abc, abc, 3 * count, tw.inv.as<fr_t>(), shift, log_n, tw.pass_bits[log_n], st);
-  const Fr ninv = Fr::from_u64(n).inv();
-  const Fr c_odd = ninv * host_root(log_n + 1);
-  k_coset_scale<<<dim3(blocks_for(n), 3 * count), 256, 0, st>>>(abc, tw.fwd.as<fr_t>(), shift,
-                                                                log_n, to_dev(ninv), to_dev(c_odd));
+  dif(abc, abc, abc, 3 * count, tw.inv.as<fr_t>(), shift, log_n, tw.pass_bits[log_n], st);
+  k_coset_scale<<<dim3(blocks_for(n), count), kElemThreads, 0, st>>>(
+      abc, tw.fwd.as<fr_t>(), shift, log_n, to_dev(host_root(log_n + 1)));
   ZK_LAUNCHED();
   dit(abc, 3 * count, tw.fwd.as<fr_t>(), shift, log_n, tw.pass_bits[log_n], st);
   k_h_final<<<dim3(blocks_for(n), count), 256, 0, st>>>(ha, n);
@@ -457,7 +592,7 @@ namespace {
 
 struct HJobDev {
   fr_t *a, *b, *c, *h;
-  fr_t c_even, c_odd;  // coset factors: 1/N and omega_2N / N
+  fr_t w2n;  // omega_2N
   uint32_t L, np, shift, elem_blocks;
   uint32_t pass_blocks[kMaxHPasses];  // tiles per array of pass i (bit ranges low -> high)
   uint8_t lo[kMaxHPasses], k[kMaxHPasses], log_g[kMaxHPasses];
@@ -477,7 +612,7 @@ __host__ __device__ inline uint32_t h_items(const HJobDev& J, uint32_t s) {
   const uint32_t np = J.np;
   if (s == 0 || s == 2 * np + 2) return J.elem_blocks;
   if (s <= np) return 3 * J.pass_blocks[np - s];
-  if (s == np + 1) return 3 * J.elem_blocks;
+  if (s == np + 1) return J.elem_blocks;  // all three vectors
   if (s <= 2 * np + 1) return 3 * J.pass_blocks[s - np - 2];
   return 0;
 }
@@ -540,10 +675,9 @@ __global__ void __launch_bounds__(kPassThreads) k_hpoly_persistent(const __grid_
       pass_tile<false, true>(x, x, local % nb, p.tw_inv, J.shift, J.L, J.lo[pi], J.k[pi],
                              J.log_g[pi], sm);
     } else if (st == np + 1) {
-      const uint32_t arr = local / J.elem_blocks;
-      fr_t* x = arr == 0 ? J.a : (arr == 1 ? J.b : J.c);
-      const size_t i = (size_t)(local % J.elem_blocks) * kPassThreads + threadIdx.x;
-      if (i < n) coset_elem<true>(x, i, p.tw_fwd, J.shift, J.L, J.c_even, J.c_odd);
+      fr_t* const v[3] = {J.a, J.b, J.c};
+      const size_t i = (size_t)local * kPassThreads + threadIdx.x;
+      if (i < n) coset_elem<true>(v, i, p.tw_fwd, J.shift, J.L, J.w2n);
     } else if (st <= 2 * np + 1) {
       const uint32_t pi = st - np - 2, nb = J.pass_blocks[pi];
       const uint32_t arr = local / nb;
@@ -565,7 +699,7 @@ __global__ void __launch_bounds__(kPassThreads) k_hpoly_persistent(const __grid_
 // Blocks per SM the persistent H pipeline takes at most: it runs beside the
 // MSM chains of the same group, so it leaves them room
 #ifndef ZK_HPOLY_PER_SM
-#define ZK_HPOLY_PER_SM 2
+#define ZK_HPOLY_PER_SM 4
 #endif
 int hpoly_grid() {
   static const int g = [] {
@@ -625,9 +759,7 @@ void hpoly_multi(NttTables& tw, int count, const HJob* jobs, uint32_t* sync, cud
       J.log_g[i] = (uint8_t)log_g;
       J.pass_blocks[i] = (uint32_t)(groups >> log_g);
     }
-    const Fr ninv = Fr::from_u64(n).inv();
-    J.c_even = to_dev(ninv);
-    J.c_odd = to_dev(ninv * host_root(L + 1));
+    J.w2n = to_dev(host_root(L + 1));
     nsteps = nsteps > 2u * np + 3u ? nsteps : 2u * np + 3u;
     units += 6.0 * np * (double)n;
   }

@@ -12,7 +12,8 @@
 // and writes back.  Decimation-in-frequency passes take natural order to
 // bit-reversed order, decimation-in-time passes the reverse, so the H
 // pipeline (INTT -> coset shift -> NTT) never permutes: it keeps coefficients
-// in bit-reversed order between the two transforms.
+// in bit-reversed order between the two transforms.  A transform on its own
+// is DIF passes whose last one stores in natural order.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -27,7 +28,7 @@ constexpr int kMaxLogN = 27;  // Fr 2-adicity is 28; H needs omega_2n
 // Twiddle tables tw[e] = w^e (forward) and w^-e (inverse), e < 2^(lmax-1),
 // w a primitive 2^lmax-th root.  Smaller transforms read them with a stride.
 // pass_bits[L]: largest radix (2^bits, 4..8) of one shared-memory pass for
-// transforms of 2^L points (a tunable; kernels hold tiles of 1024 points).
+// transforms of 2^L points (a tunable; kernels hold tiles of 512 points).
 constexpr int kMaxPassBits = 8;
 struct NttTables {
   int lmax = -1;
