@@ -20,6 +20,8 @@
 #pragma once
 #include <cstdint>
 
+#include "field_inv.cuh"
+
 namespace zk {
 
 struct FpCfg {
@@ -30,6 +32,8 @@ struct FpCfg {
                                       0x7879462cu, 0x666ea36fu, 0x9a07df2fu, 0x0e0a77c1u};
   static constexpr uint32_t R2[8] = {0x538afa89u, 0xf32cfc5bu, 0xd44501fbu, 0xb5e71911u,
                                      0x0a417ff6u, 0x47ab1effu, 0xcab8351fu, 0x06d89f71u};
+  static constexpr uint32_t R3[8] = {0xda1530dfu, 0xb1cd6dafu, 0xa7283db6u, 0x62f210e6u,
+                                     0x0ada0afbu, 0xef7f0b0cu, 0x2d592544u, 0x20fd6e90u};
 };
 
 struct FrCfg {
@@ -40,6 +44,8 @@ struct FrCfg {
                                       0x7879462eu, 0x666ea36fu, 0x9a07df2fu, 0x0e0a77c1u};
   static constexpr uint32_t R2[8] = {0xae216da7u, 0x1bb8e645u, 0xe35c59e3u, 0x53fe3ab1u,
                                      0x53bb8085u, 0x8c49833du, 0x7f4e44a5u, 0x0216d0b1u};
+  static constexpr uint32_t R3[8] = {0xb4bf0040u, 0x5e94d8e1u, 0x1cfbb6b8u, 0x2a489cbeu,
+                                     0xa19fcfedu, 0x893cc664u, 0x7fcc657cu, 0x0cf8594bu};
 };
 
 template <class C>
@@ -540,24 +546,21 @@ __device__ __forceinline__ fe<C> fe_from_mont(const fe<C>& a) {
   return fe_redc<C>(T);
 }
 
-// a^e for a small public exponent given as 8 x u32 limbs (square-and-multiply)
+// Inverse by division steps (field_inv.cuh); inv(0) = 0 like the reference's
+// Bernstein-Yang inversion (include/fp_bn254.cuh:720-773).  For a = x R the
+// division steps give x^-1 R^-1, and one product by R^3 makes it x^-1 R.
+// About 15 K instructions against ~100 K for a^(m-2).
 template <class C>
-__device__ __forceinline__ fe<C> fe_pow(const fe<C>& a, const uint32_t* e) {
-  fe<C> acc = fe_one<C>();
-  for (int i = 255; i >= 0; i--) {
-    acc = fe_sqr(acc);
-    if ((e[i >> 5] >> (i & 31)) & 1) acc = acc * a;
-  }
-  return acc;
+__device__ __noinline__ fe<C> fe_inv_call(fe<C> a) {
+  const uint32_t m[8] = {C::P0, C::P1, C::P2, C::P3, C::P4, C::P5, C::P6, C::P7};
+  const fe<C> r3{{C::R3[0], C::R3[1], C::R3[2], C::R3[3], C::R3[4], C::R3[5], C::R3[6], C::R3[7]}};
+  fe<C> t;
+  inv_divsteps(a.v, m, C::INV & (uint32_t)kInvMask, t.v);
+  return t * r3;
 }
-
-// Inverse by Fermat's little theorem (a^(m-2)); inv(0) = 0 like the reference's
-// Bernstein-Yang inversion (include/fp_bn254.cuh:720-773).  Only used off the
-// hot loops (window results, affine conversion of single points).
 template <class C>
 __device__ __forceinline__ fe<C> fe_inv(const fe<C>& a) {
-  const uint32_t e[8] = {C::P0 - 2u, C::P1, C::P2, C::P3, C::P4, C::P5, C::P6, C::P7};
-  return fe_pow(a, e);
+  return fe_inv_call<C>(a);
 }
 
 // ------------------------------------------------------------------- Fp2
@@ -723,10 +726,27 @@ __device__ __forceinline__ fp2_t fe_sqr(const fp2_t& a) {
 __device__ __forceinline__ fp2_t fe_dbl(const fp2_t& a) { return {a.c0 + a.c0, a.c1 + a.c1}; }
 __device__ __forceinline__ bool fe_is_zero(const fp2_t& a) { return fe_is_zero(a.c0) && fe_is_zero(a.c1); }
 __device__ __forceinline__ fp2_t fe_neg(const fp2_t& a) { return {fe_neg(a.c0), fe_neg(a.c1)}; }
-__device__ __forceinline__ fp2_t fe_inv(const fp2_t& a) {
-  fp_t n = a.c0 * a.c0 + a.c1 * a.c1;
-  fp_t ni = fe_inv(n);
-  return {a.c0 * ni, fe_neg(a.c1) * ni};
+// Norm to Fp and the inverse from the inverse norm: 1/a = conj(a) / N(a) with
+// N(a) = c0^2 + c1^2 (nonzero for a nonzero, as -1 is not a square mod p).
+// The sum of the two unreduced squares is below 2 p^2, one reduction.  In Fp
+// the norm is the element itself, so code written over norms shares
+// inversions in Fp for both groups.
+static __device__ __noinline__ fp_t fp2_norm_call(fp2_t a) {
+  uint32_t x[16], w[16];
+  fe_sqr_wide(a.c0.v, x);
+  fe_sqr_wide(a.c1.v, w);
+  add_16(x, w);
+  return fe_redc<FpCfg>(x);
+}
+__device__ __forceinline__ fp_t fe_norm(const fp_t& a) { return a; }
+__device__ __forceinline__ fp_t fe_norm(const fp2_t& a) { return fp2_norm_call(a); }
+__device__ __forceinline__ fp_t fe_inv_of(const fp_t&, const fp_t& ni) { return ni; }
+__device__ __forceinline__ fp2_t fe_inv_of(const fp2_t& a, const fp_t& ni) {
+  return {a.c0 * ni, fe_neg(a.c1 * ni)};
+}
+__device__ __forceinline__ fp2_t fe_inv(const fp2_t& a) { return fe_inv_of(a, fe_inv(fe_norm(a))); }
+__device__ __forceinline__ bool fe_eq(const fp2_t& a, const fp2_t& b) {
+  return fe_eq(a.c0, b.c0) && fe_eq(a.c1, b.c1);
 }
 
 template <class T>

@@ -21,7 +21,6 @@ constexpr uint32_t kNeg = 0x80000000u;
 // pairs per block in the bucket-reduction block passes
 template <class F>
 constexpr int red_pairs() { return sizeof(F) == 64 ? 64 : 128; }
-constexpr int red_pairs(bool g2) { return g2 ? 64 : 128; }
 // nodes per block (a quad each) of the later levels of the segmented reduction
 constexpr int lvl_nodes(bool g2) { return g2 ? 64 : 128; }
 template <class F>
@@ -39,12 +38,16 @@ struct Shape {
   size_t entries;        // W*B + 1 scan entries (last = total)
   size_t records;        // W*n upper bound on sorted records
   int k0, k1, chunk;
+  size_t affine;         // tiles of level 0 as batched affine additions (G2; 0: XYZZ)
   int levels;            // segmented-reduction levels (>= 1)
   size_t lvl_records[24];
   size_t lvl_blocks[24];
   int lvl_k[24];         // records per thread of each level
   size_t J;              // bucket-reduction level-1 chunks per window
 };
+
+size_t affine_tiles(size_t records, size_t buckets);
+size_t affine_scratch(size_t records, size_t tiles);
 
 // n: points (summed over instances for fixed-base multi-instance MSMs)
 Shape make_shape(size_t n, bool g2, const MsmConfig& cfg, bool fixed = false, int inst = 1) {
@@ -68,6 +71,14 @@ Shape make_shape(size_t n, bool g2, const MsmConfig& cfg, bool fixed = false, in
   size_t rec = s.records;
   int per_thread = s.k0;
   s.levels = 0;
+  s.affine = g2 ? affine_tiles(s.records, (size_t)s.Wk * s.B) : 0;
+  if (s.affine) {
+    s.lvl_records[0] = rec;
+    s.lvl_blocks[0] = s.affine;
+    s.levels = 1;
+    rec = 2 * s.affine;
+    per_thread = s.k1;
+  }
   while (true) {
     // a level that fits one block spreads its records over every thread
     // (its depth is the per-thread run plus the block tree)
@@ -99,6 +110,7 @@ struct Layout {
   xyzz<F>* rrun[2];   // bucket-reduction (run, acc) pairs, ping-pong
   xyzz<F>* racc[2];
   xyzz<F>* outua;     // 2 * W: U_0..U_{W-1}, A_0..A_{W-1}
+  unsigned char* aff;  // affine accumulation: scratch of its resident blocks
   size_t bytes;
 };
 
@@ -110,7 +122,7 @@ Layout<F> carve(void* base, const Shape& s) {
   L.tileq = L.counts + s.entries;
   L.cursor = cv.take<uint32_t>(s.entries);
   L.tiles = cv.take<uint32_t>(scan::tile_count(s.entries) + 1);
-  L.srec = cv.take<uint2>(s.records);
+  L.srec = cv.take<uint2>(s.records + 1);
   L.buckets = cv.take<xyzz<F>>((size_t)s.Wk * s.B);
   size_t pmax[2] = {1, 1};
   for (int l = 1; l < s.levels; l++) pmax[l & 1] = std::max(pmax[l & 1], s.lvl_records[l]);
@@ -124,6 +136,7 @@ Layout<F> carve(void* base, const Shape& s) {
   L.rrun[1] = cv.take<xyzz<F>>((size_t)s.Wk * j2);
   L.racc[1] = cv.take<xyzz<F>>((size_t)s.Wk * j2);
   L.outua = cv.take<xyzz<F>>((size_t)s.Wk * 2);
+  L.aff = cv.take<unsigned char>(s.affine ? affine_scratch(s.records, s.affine) : 0);
   L.bytes = cv.off + 256;
   return L;
 }
@@ -485,6 +498,547 @@ __global__ void __launch_bounds__(seg_threads<F>()) k_msm_accum0_queue(
   }
 }
 
+// ------------------------------------------- batched affine accumulation
+// A large G2 MSM's sorted list holds long runs of one bucket.  They are added
+// pairwise in affine coordinates before the XYZZ accumulation sees them.  An
+// affine addition costs two Fp2 products, a square and an inversion, and
+// Montgomery's trick over the norms in Fp makes the inversion five Fp products
+// and a norm plus a shared one: about 3000 multiply instructions against 5400
+// of the mixed XYZZ addition, with half the live registers (16 warps per SM
+// instead of 8).
+//
+// A block takes T * S consecutive records, S per thread.  In a round every
+// thread pairs neighbours of the same run among its own points:
+//   forward: the norm of each pair's denominator joins the thread's running
+//     product (the product before it is stored);
+//   the block's T products are inverted by one warp, a lane for each column
+//     of T / 32 of them (32 inversions at the cost of one);
+//   backward: every pair with its own inverse; sums and then the left-over
+//     points are written compactly into the other of two slot buffers.
+// Rounds go on while they pay for their inversions.  The few points left of
+// each run go through the XYZZ accumulation and the block tree.
+//
+// Fixed-base 2^20 points (20-bit windows, runs of 26): 5.6 ms against 7.5 ms
+// for the XYZZ accumulation, 2^18: 1.8 against 2.5.  Bound by the latency of
+// the gathers and of the scattered slots (about 700 B of DRAM traffic per
+// record), not by the multiply pipe (57 % busy).  For the same reason G1 keeps
+// the XYZZ accumulation, whose additions are 2.5 times cheaper: there the
+// rounds measured 2.71 against 2.70 ms.  Copying pairs to shared memory ahead
+// (cp.async) was slower: scattered 16-byte copies cost a shared-memory
+// wavefront each.
+//
+// The run structure is kept as bit masks per sub-segment of 64 points: bit j
+// of `ends` is set when point j is the last of its run.  A round about halves
+// the points, and the slots are sized for that; a block with runs too short
+// for it (or for one round to pay) skips the rounds.
+constexpr int kAffT = 128;      // threads per block
+constexpr int kSub = 64;        // points per sub-segment
+constexpr int kAffMaxSub = 3;   // sub-segments per thread: S <= 192
+constexpr int kAffMinS = 32;    // records per thread, at least
+constexpr int kAffLeast = 8;    // additions left per thread for a round to pay
+constexpr uint32_t kAffUntouched = 1u << 31;  // state: points still the table's
+constexpr uint32_t kAffFirst = 1u << 30;      // state: points in slot buffer 1
+
+// Layout of one resident block's scratch, interleaved by thread, for at most
+// S records per thread.
+struct AffShape {
+  int nsub;       // sub-segments per thread
+  int slots[2];   // slots per sub-segment: buffer 1 takes the first round's
+                  // results, buffer 0 the second's, and so on in turn
+  uint32_t pre;   // byte offsets of the pairs' prefixes and norms,
+  uint32_t mask;  // of the masks
+  uint32_t state; // and of the final state
+  uint32_t bytes;
+};
+__host__ __device__ inline AffShape aff_shape(int S) {
+  AffShape a;
+  a.nsub = (S + kSub - 1) / kSub;
+  const int sub = S < kSub ? S : kSub;
+  a.slots[0] = sub / 2;
+  a.slots[1] = sub - sub / 4;
+  const uint32_t buf = (uint32_t)(a.nsub * kAffT) * 2 * sizeof(fp2_t);
+  a.pre = buf * (a.slots[0] + a.slots[1]);
+  a.mask = a.pre + (uint32_t)(a.nsub * (sub / 2) * kAffT) * 2 * sizeof(fp_t);
+  a.state = a.mask + (uint32_t)(a.nsub * 3 * kAffT) * sizeof(uint64_t);
+  a.bytes = a.state + kAffT * sizeof(uint32_t);
+  return a;
+}
+static_assert(kAffMaxSub * kSub < 256 && kAffMinS % 4 == 0, "layout of the affine scratch");
+
+// Records per thread (even) of a list of `total` over ntiles tiles: spread
+// evenly by the actual number, so skewed scalars, whose zero digits make no
+// records, leave no tile idle.
+__host__ __device__ inline int aff_span(size_t total, uint32_t ntiles) {
+  const size_t lanes = (size_t)ntiles * kAffT;
+  const int S = ((int)((total + lanes - 1) / lanes) + 1) & ~1;
+  return S < kAffMinS ? kAffMinS : S;
+}
+
+struct AffScratch {
+  unsigned char* base;
+  const AffShape& a;
+  __device__ __forceinline__ fp2_t* slot(int buf, int h, int j) const {
+    const int row = h * a.slots[buf] + j + (buf ? a.nsub * a.slots[0] : 0);
+    return reinterpret_cast<fp2_t*>(base) + 2 * (uint32_t)(row * kAffT + threadIdx.x);
+  }
+  // prefix product and norm of pair k
+  __device__ __forceinline__ fp_t* pair(int k) const {
+    return reinterpret_cast<fp_t*>(base + a.pre) + 2 * (uint32_t)(k * kAffT + threadIdx.x);
+  }
+  // which: 0 run ends now, 1 run ends of the sorted records, 2 pairs of the round
+  __device__ __forceinline__ uint64_t& mask(int h, int which) const {
+    return reinterpret_cast<uint64_t*>(base + a.mask)[(3 * h + which) * kAffT + threadIdx.x];
+  }
+  // points of each sub-segment (8 bits each) and the kAff* flags
+  __device__ __forceinline__ uint32_t& state() const {
+    return reinterpret_cast<uint32_t*>(base + a.state)[threadIdx.x];
+  }
+};
+
+__device__ __forceinline__ uint64_t aff_low(int n) { return n >= 64 ? ~0ull : (1ull << n) - 1; }
+// Bit j set when points j and j + 1 of a sub-segment of cnt points belong to
+// one run.
+__device__ __forceinline__ uint64_t aff_links(uint64_t ends, int cnt) {
+  return ~ends & aff_low(cnt);
+}
+// The pairs (j, j + 1) of the links, from the top of each run down, as the
+// bits of their first points.
+__device__ __forceinline__ uint64_t aff_pairs(uint64_t links) {
+  uint64_t m = 0;
+  while (links) {
+    const int j = 63 - __clzll((long long)links);
+    links &= j ? aff_low(j - 1) : 0;
+    m |= 1ull << j;
+  }
+  return m;
+}
+// `ends` after the pairs m became one point each (their first points' bits,
+// which are clear, drop out).
+__device__ __forceinline__ uint64_t aff_squeeze(uint64_t ends, uint64_t m) {
+  while (m) {
+    const int j = 63 - __clzll((long long)m);
+    m ^= 1ull << j;
+    ends = (ends & aff_low(j)) | ((ends >> 1) & ~aff_low(j));
+  }
+  return ends;
+}
+
+// How two affine points add: in general, as a doubling, or without any
+// arithmetic (one of them or the sum is the point at infinity).
+enum AffKind { kAffGeneral, kAffDouble, kAffTakeSecond, kAffTakeFirst, kAffInfinity };
+template <class LoadY>
+__device__ __forceinline__ int aff_kind(const fp2_t& x1, const fp2_t& x2, const fp2_t& d,
+                                        LoadY load_y) {
+  const bool zd = fe_is_zero(d), z1 = fe_is_zero(x1), z2 = fe_is_zero(x2);
+  if (!(zd || z1 || z2)) return kAffGeneral;
+  const fp2_t y1 = load_y(0), y2 = load_y(1);
+  if (z1 && fe_is_zero(y1)) return kAffTakeSecond;
+  if (z2 && fe_is_zero(y2)) return kAffTakeFirst;
+  if (!zd) return kAffGeneral;
+  return fe_eq(y1, y2) && !fe_is_zero(y1) ? kAffDouble : kAffInfinity;
+}
+
+// Inverts the kAffT products in place (one warp; none of them is zero).
+__device__ __forceinline__ void aff_invert(fp_t* tot) {
+  constexpr int R = kAffT / 32;
+  fp_t* v = tot + (threadIdx.x & 31);
+  fp_t pre[R];
+  pre[0] = v[0];
+#pragma unroll
+  for (int i = 1; i < R; i++) pre[i] = pre[i - 1] * v[32 * i];
+  fp_t inv = fe_inv(pre[R - 1]);
+#pragma unroll
+  for (int i = R - 1; i > 0; i--) {
+    const fp_t x = v[32 * i];
+    v[32 * i] = inv * pre[i - 1];
+    inv = inv * x;
+  }
+  v[0] = inv;
+}
+
+// The points of one thread: the table's (with the record's sign) before the
+// first round, the thread's slots afterwards.
+template <bool kFixed>
+struct AffPoints {
+  const uint2* rec;  // the thread's sorted records
+  const PointSrc<fp2_t>& src;
+  const AffScratch& scr;
+  bool first;
+  int buf;  // slot buffer that holds the points
+  __device__ __forceinline__ const fp2_t* at(const uint2& r, bool y) const {
+    const size_t idx = r.y & ~kNeg;
+    if (kFixed) return src.table[r.x >> src.bshift] + 2 * idx + y;
+    return (y ? src.y : src.x) + idx * src.stride;
+  }
+  __device__ __forceinline__ uint2 record(int h, int j) const { return rec[h * kSub + j]; }
+  __device__ __forceinline__ fp2_t x(int h, int j) const {
+    return ld_pod(first ? at(record(h, j), false) : scr.slot(buf, h, j));
+  }
+  __device__ __forceinline__ fp2_t y(int h, int j) const {
+    if (!first) return ld_pod(scr.slot(buf, h, j) + 1);
+    const uint2 r = record(h, j);
+    const fp2_t v = ld_pod(at(r, true));
+    return r.y & kNeg ? fe_neg(v) : v;
+  }
+};
+
+// Walks the pairs of the thread's sub-segments, from the last one down or
+// from the first one up.
+template <bool kDown>
+struct AffWalk {
+  const AffScratch& scr;
+  int nsub, h, j = 0;  // h: current sub-segment; -1 past the last pair
+  uint64_t m;
+  __device__ __forceinline__ AffWalk(const AffScratch& scr, int n) : scr(scr), nsub(n) {
+    h = kDown ? n - 1 : 0;
+    m = scr.mask(h, 2);
+  }
+  __device__ __forceinline__ void next() {
+    while (!m && h >= 0) {
+      h = kDown ? h - 1 : (h + 1 < nsub ? h + 1 : -1);
+      if (h >= 0) m = scr.mask(h, 2);
+    }
+    if (h < 0) return;
+    j = kDown ? 63 - __clzll((long long)m) : __ffsll((long long)m) - 1;
+    m ^= 1ull << j;
+  }
+};
+
+// The rounds of tile tile0 + blockIdx.x.  kBlocks per SM: 3 (168 registers,
+// ~350 bytes a thread spilled, as many tail blocks fit) or 4 (128 registers,
+// ~650 bytes spilled, a third more scratch); see affine_blocks.
+template <bool kFixed, int kBlocks>
+__global__ void __launch_bounds__(kAffT, kBlocks) k_msm_affine(
+    const uint2* __restrict__ srec, const uint32_t* __restrict__ total_p,
+    const __grid_constant__ PointSrc<fp2_t> src, const __grid_constant__ AffShape shape,
+    unsigned char* __restrict__ scratch, uint32_t tile0, uint32_t ntiles) {
+  __shared__ fp_t tot[kAffT];
+  __shared__ uint32_t left[kAffT / 32];
+  const size_t total = *total_p;
+  const int S = aff_span(total, ntiles);
+  const size_t b = tile0 + blockIdx.x;
+  const AffScratch scr{scratch + (size_t)blockIdx.x * shape.bytes, shape};
+  const int t = threadIdx.x;
+  const size_t s = min((b * kAffT + t) * S, total);
+  const int len = (int)min((size_t)S, total - s);
+  const int nsub = (S + kSub - 1) / kSub;
+  AffPoints<kFixed> pts{srec + s, src, scr, true, 0};
+  uint32_t cnts = 0;  // points of each sub-segment, 8 bits each
+
+  int links = 0;  // additions left
+  bool fits = true;
+  for (int h = 0; h < nsub; h++) {
+    const int cnt = min(max(len - h * kSub, 0), kSub);
+    // s is even: two records (16 bytes) at a time; the list has room for the
+    // word after its last record
+    const uint4* r = reinterpret_cast<const uint4*>(srec + s + h * kSub);
+    uint64_t ends = 0;
+    uint32_t key = kInvalid;  // of the record before
+    for (int j = 0; j < cnt; j += 2) {
+      const uint4 v = r[j / 2];
+      if (j) ends |= (uint64_t)(v.x != key) << (j - 1);
+      ends |= (uint64_t)(v.z != v.x) << j;
+      key = v.z;
+    }
+    if (cnt) ends = (ends | 1ull << (cnt - 1)) & aff_low(cnt);
+    const uint64_t C = aff_links(ends, cnt), M = aff_pairs(C);
+    scr.mask(h, 0) = ends;
+    scr.mask(h, 1) = ends;
+    scr.mask(h, 2) = M;
+    cnts |= (uint32_t)cnt << (8 * h);
+    links += __popcll(C);
+    const int o1 = cnt - __popcll(M);
+    const int o2 = o1 - __popcll(aff_pairs(aff_links(aff_squeeze(ends, M), o1)));
+    fits = fits && o1 <= shape.slots[1] && o2 <= shape.slots[0];
+  }
+  const int lanes = __syncthreads_count(len > 0);
+
+  for (uint32_t round = 0;; round++) {
+    const uint32_t wsum = __reduce_add_sync(0xffffffffu, (uint32_t)links);
+    if ((t & 31) == 0) left[t >> 5] = wsum;
+    if (!__syncthreads_and(fits)) break;
+    uint32_t sum = 0;
+#pragma unroll
+    for (int w = 0; w < kAffT / 32; w++) sum += left[w];
+    if (!sum || sum < (uint32_t)(kAffLeast * lanes)) break;
+
+    fp_t run = fe_one<FpCfg>();
+    int k = 0;
+    {
+      // a pair has only a norm and a product here, too short to hide its
+      // gathers behind: two pairs are read at a time
+      constexpr int kAhead = 2;
+      AffWalk<true> w(scr, nsub);
+      while (w.h >= 0) {
+        int h[kAhead], j[kAhead];
+        fp2_t x1[kAhead], x2[kAhead];
+        uint2 r1[kAhead], r2[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; i++) {
+          w.next();
+          h[i] = w.h;
+          j[i] = w.j;
+          if (pts.first && w.h >= 0) {
+            r1[i] = pts.record(w.h, w.j);
+            r2[i] = pts.record(w.h, w.j + 1);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kAhead; i++) {
+          if (h[i] < 0) continue;
+          x1[i] = ld_pod(pts.first ? pts.at(r1[i], false) : scr.slot(pts.buf, h[i], j[i]));
+          x2[i] = ld_pod(pts.first ? pts.at(r2[i], false) : scr.slot(pts.buf, h[i], j[i] + 1));
+        }
+#pragma unroll
+        for (int i = 0; i < kAhead; i++) {
+          if (h[i] < 0) break;
+          fp2_t d = x2[i] - x1[i];
+          const int kind = aff_kind(x1[i], x2[i], d, [&](int q) { return pts.y(h[i], j[i] + q); });
+          if (kind == kAffDouble) d = fe_dbl(pts.y(h[i], j[i]));
+          fp_t n = fe_one<FpCfg>();
+          if (kind <= kAffDouble) n = fe_norm(d);
+          st_pod(scr.pair(k), run);
+          st_pod(scr.pair(k) + 1, n);
+          run = run * n;
+          k++;
+        }
+      }
+    }
+    tot[t] = run;
+    __syncthreads();
+    // the inverting warp rotates, so that blocks that share an SM load its
+    // four schedulers evenly
+    if ((t >> 5) == (int)((round + b) % (kAffT / 32))) aff_invert(tot);
+    __syncthreads();
+    fp_t inv = tot[t];
+    const int ob = pts.buf ^ 1;
+    {
+      AffWalk<false> w(scr, nsub);
+      uint2 ra{}, rb{};  // the pair's records, read a step ahead (first round)
+      const auto next = [&] {
+        w.next();
+        if (pts.first && w.h >= 0) {
+          ra = pts.record(w.h, w.j);
+          rb = pts.record(w.h, w.j + 1);
+        }
+      };
+      next();
+      while (w.h >= 0) {
+        const int h = w.h, j = w.j;
+        k--;
+        const fp_t pre = ld_pod(scr.pair(k)), n = ld_pod(scr.pair(k) + 1);
+        fp2_t x1, y1, x2, num;
+        if (pts.first) {
+          x1 = ld_pod(pts.at(ra, false));
+          y1 = ld_pod(pts.at(ra, true));
+          x2 = ld_pod(pts.at(rb, false));
+          num = ld_pod(pts.at(rb, true));
+          if (ra.y & kNeg) y1 = fe_neg(y1);
+          if (rb.y & kNeg) num = fe_neg(num);
+        } else {
+          const fp2_t* q = scr.slot(pts.buf, h, j);
+          x1 = ld_pod(q);
+          y1 = ld_pod(q + 1);
+          x2 = ld_pod(q + 2 * kAffT);
+          num = ld_pod(q + 2 * kAffT + 1);
+        }
+        fp2_t* const out = scr.slot(ob, h, j - __popcll(scr.mask(h, 2) & aff_low(j)));
+        next();
+        fp2_t d = x2 - x1;
+        const int kind = aff_kind(x1, x2, d, [&](int q) { return q ? num : y1; });
+        fp2_t xo = x2, yo = num;
+        if (kind <= kAffDouble) {
+          if (kind == kAffDouble) {
+            d = fe_dbl(y1);
+            num = fe_triple(fe_sqr(x1));
+          } else {
+            num = num - y1;
+          }
+          const fp_t ni = inv * pre;
+          inv = inv * n;
+          const fp2_t lam = num * fe_inv_of(d, ni);
+          xo = fe_sqr(lam) - x1 - x2;
+          yo = lam * (x1 - xo) - y1;
+        } else if (kind == kAffTakeFirst) {
+          xo = x1;
+          yo = y1;
+        } else if (kind == kAffInfinity) {
+          xo = fe_zero_of<fp2_t>();
+          yo = fe_zero_of<fp2_t>();
+        }
+        st_pod(out, xo);
+        st_pod(out + 1, yo);
+      }
+    }
+    // the points without a partner move over, and the masks follow
+    links = 0;
+    for (int h = 0; h < nsub; h++) {
+      const uint64_t ends = scr.mask(h, 0), M = scr.mask(h, 2);
+      const int cnt = (cnts >> (8 * h)) & 255;
+      uint64_t alone = ~(M | M << 1) & aff_low(cnt);
+      while (alone) {
+        const int j = __ffsll((long long)alone) - 1;
+        alone &= alone - 1;
+        const fp2_t x = pts.x(h, j), y = pts.y(h, j);
+        fp2_t* const out = scr.slot(ob, h, j - __popcll(M & aff_low(j)));
+        st_pod(out, x);
+        st_pod(out + 1, y);
+      }
+      const int o = cnt - __popcll(M);
+      const uint64_t e = aff_squeeze(ends, M), C = aff_links(e, o);
+      scr.mask(h, 0) = e;
+      scr.mask(h, 2) = aff_pairs(C);
+      cnts = (cnts & ~(255u << (8 * h))) | ((uint32_t)o << (8 * h));
+      links += __popcll(C);
+    }
+    pts.first = false;
+    pts.buf = ob;
+  }
+  scr.state() = cnts | (pts.first ? kAffUntouched : 0) | (pts.buf ? kAffFirst : 0);
+}
+
+// The XYZZ accumulation of the points the rounds of a tile left, and the
+// block tree over its threads.  A kernel of its own: its register need would
+// halve the rounds' residency.  Beside four round blocks per SM the tail
+// runs as two waves of two (255 registers): 7.78 against 7.95 ms for a 2^20
+// MSM with three spilling ones.
+template <bool kFixed, int kBlocks>
+__global__ void __launch_bounds__(kAffT, kBlocks == 3 ? 3 : 1) k_msm_affine_tail(
+    const uint2* __restrict__ srec, const uint32_t* __restrict__ total_p,
+    const __grid_constant__ PointSrc<fp2_t> src, const __grid_constant__ AffShape shape,
+    unsigned char* __restrict__ scratch, xyzz<fp2_t>* __restrict__ buckets,
+    uint32_t* __restrict__ okey, xyzz<fp2_t>* __restrict__ opt, uint32_t tile0, uint32_t ntiles) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  SegNode<fp2_t>* sm = reinterpret_cast<SegNode<fp2_t>*>(smem);
+  const size_t total = *total_p;
+  const int S = aff_span(total, ntiles);
+  const size_t b = tile0 + blockIdx.x;
+  const AffScratch scr{scratch + (size_t)blockIdx.x * shape.bytes, shape};
+  const int t = threadIdx.x;
+  const size_t bstart = min(b * kAffT * S, total);
+  const size_t bend = min(bstart + (size_t)kAffT * S, total);
+  const size_t s = min(bstart + (size_t)t * S, total);
+  const int nsub = (S + kSub - 1) / kSub;
+  const uint32_t state = scr.state();
+  const AffPoints<kFixed> pts{srec + s, src, scr, (state & kAffUntouched) != 0,
+                              (state & kAffFirst) ? 1 : 0};
+  SegNode<fp2_t>& nd = sm[t];
+  nd.fk = nd.lk = kInvalid;
+  nd.single = 1;
+  xyzz<fp2_t> acc = xyzz_inf<fp2_t>();
+  uint32_t cur = kInvalid;
+  // a step of the loop ends at a point that has to be added: the points that
+  // only begin a run are passed on the way, so the lanes add together
+  int h = -1, j = 0, cnt = 0;
+  uint64_t ends = 0, runs = 0;
+  bool begins = true;
+  for (;;) {
+    bool add = false;
+    fp2_t x, y;
+    while (!add) {
+      while (j >= cnt && h + 1 < nsub) {
+        h++;
+        j = 0;
+        cnt = (state >> (8 * h)) & 127;
+        ends = scr.mask(h, 0);
+        runs = scr.mask(h, 1);
+        begins = true;
+      }
+      if (j >= cnt) break;
+      if (begins) {
+        const uint32_t key = srec[s + h * kSub + __ffsll((long long)runs) - 1].x;
+        runs &= runs - 1;
+        if (key != cur) {
+          seg_close(nd, acc, cur, buckets);
+          cur = key;
+          acc = xyzz_inf<fp2_t>();
+        }
+      }
+      begins = (ends >> j) & 1;
+      x = pts.x(h, j);
+      y = pts.y(h, j);
+      j++;
+      if (fe_is_zero(x) && fe_is_zero(y)) continue;
+      if (xyzz_is_inf(acc))
+        acc = {x, y, fe_one_of<fp2_t>(), fe_one_of<fp2_t>()};
+      else
+        add = true;
+    }
+    if (!add) break;
+    acc = xyzz_madd(acc, x, y);
+  }
+  seg_close(nd, acc, cur, buckets);
+  const uint32_t key_before = bstart && bstart < bend ? srec[bstart - 1].x : kInvalid;
+  const uint32_t key_after = bend < total ? srec[bend].x : kInvalid;
+  seg_block_finish<fp2_t, kAffT>(sm, key_before, key_after, buckets, okey, opt, b);
+}
+
+// Blocks of the rounds the device holds at once: one wave.
+template <int kBlocks>
+size_t affine_grid_of() {
+  static const int g = [] {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_msm_affine<true, kBlocks>, kAffT,
+                                                      0) != cudaSuccess) {
+      (void)cudaGetLastError();
+      per_sm = 1;
+    }
+    return std::max(1, per_sm) * device_sm_count();
+  }();
+  return (size_t)g;
+}
+size_t affine_grid(int blocks) { return blocks == 3 ? affine_grid_of<3>() : affine_grid_of<4>(); }
+size_t affine_wave(int blocks) { return affine_grid(blocks) * kAffT * kAffMaxSub * kSub; }
+
+// Blocks per SM for a list of at most `records`: three while the list fits
+// one wave of them, four beyond.  Fixed-base 2^17 / 2^18 / 2^20 points (2.0 /
+// 3.9 / 13.6 M records against a wave of 10.9 M): 1.03 / 1.80 / 5.88 ms with
+// three, 1.14 / 1.78 / 5.60 ms with four; a 2^20 proof 20.1 against 19.4 ms.
+int affine_blocks(size_t records) { return records <= affine_wave(3) ? 3 : 4; }
+
+// Tiles of the affine accumulation for a sorted list of at most `records`
+// records in `buckets` buckets; 0 where the XYZZ accumulation takes the list:
+// runs too short, or too few records to fill two thirds of the device with
+// tiles of the least size (where the rounds' inversions stop paying: windowed
+// 2^15 points, 192 tiles, 0.59 ms XYZZ against 0.67; 2^16, 352 tiles, 1.09
+// against 0.88).
+size_t affine_tiles(size_t records, size_t buckets) {
+  if (records < 6 * buckets) return 0;
+  const int blocks = affine_blocks(records);
+  const size_t grid = affine_grid(blocks), wave = affine_wave(blocks);
+  size_t tiles = grid * ((records + wave - 1) / wave);
+  if (records < tiles * kAffT * kAffMinS) tiles = (records + kAffT * kAffMinS - 1) / (kAffT * kAffMinS);
+  return 3 * tiles < 2 * grid ? 0 : tiles;
+}
+
+size_t affine_scratch(size_t records, size_t tiles) {
+  return std::min(tiles, affine_grid(affine_blocks(records))) *
+         (size_t)aff_shape(aff_span(records, (uint32_t)tiles)).bytes;
+}
+
+// Level 0 as rounds and tail, a wave of tiles at a time (the scratch holds
+// one wave).
+template <bool kFixed, int kBlocks>
+void affine_enqueue(const uint2* srec, const uint32_t* total_p, const PointSrc<fp2_t>& src,
+                    size_t records, unsigned char* scratch, xyzz<fp2_t>* buckets, uint32_t* okey,
+                    xyzz<fp2_t>* opt, uint32_t ntiles, cudaStream_t st) {
+  constexpr size_t smem = kAffT * sizeof(SegNode<fp2_t>);
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      k_msm_affine_tail<kFixed, kBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  ZK_CUDA(attr);
+  const AffShape shape = aff_shape(aff_span(records, ntiles));
+  const uint32_t wave = (uint32_t)affine_grid(kBlocks);
+  for (uint32_t t0 = 0; t0 < ntiles; t0 += wave) {
+    const uint32_t g = std::min(wave, ntiles - t0);
+    k_msm_affine<kFixed, kBlocks><<<g, kAffT, 0, st>>>(srec, total_p, src, shape, scratch, t0,
+                                                       ntiles);
+    ZK_LAUNCHED();
+    k_msm_affine_tail<kFixed, kBlocks><<<g, kAffT, smem, st>>>(srec, total_p, src, shape, scratch,
+                                                               buckets, okey, opt, t0, ntiles);
+    ZK_LAUNCHED();
+  }
+}
+
 // Levels >= 1: records are (bucket key, XYZZ partial sum); kInvalid keys
 // carry nothing and only ever separate different keys.  A quad per node: these
 // levels are short lists, bound by the depth of their dependent additions.
@@ -805,18 +1359,29 @@ MsmResult msm_enqueue(const ScalarSrc& ss, const PointSrc<F>& ps, int inst, size
   {
     uint32_t* ok = s.levels > 1 ? L.pkey[1] : nullptr;
     ProfScope prof(g2 ? kProfAccumG2 : kProfAccumG1, (double)n_total, st);
-    if (fixed && inst > 1) {
-      const unsigned grid = (unsigned)std::min<size_t>(s.lvl_blocks[0], queue_grid<F>());
-      k_msm_accum0_queue<F, true><<<grid, seg_threads<F>(), 0, st>>>(
-          L.srec, total_p, ps, s.k0, L.buckets, ok, L.ppt[1],
-          (uint32_t)s.lvl_blocks[0], L.tileq);
-    } else if (fixed)
-      k_msm_accum0<F, true><<<(unsigned)s.lvl_blocks[0], seg_threads<F>(), 0, st>>>(
-          L.srec, total_p, ps, s.k0, L.buckets, ok, L.ppt[1]);
-    else
-      k_msm_accum0<F, false><<<(unsigned)s.lvl_blocks[0], seg_threads<F>(), 0, st>>>(
-          L.srec, total_p, ps, s.k0, L.buckets, ok, L.ppt[1]);
-    ZK_LAUNCHED();
+    const unsigned blocks = (unsigned)s.lvl_blocks[0];
+    bool affine = false;
+    if constexpr (g2) {
+      affine = s.affine != 0;
+      if (affine) {
+        const bool three = affine_blocks(s.records) == 3;
+        const auto run = fixed ? (three ? affine_enqueue<true, 3> : affine_enqueue<true, 4>)
+                               : (three ? affine_enqueue<false, 3> : affine_enqueue<false, 4>);
+        run(L.srec, total_p, ps, s.records, L.aff, L.buckets, ok, L.ppt[1], blocks, st);
+      }
+    }
+    if (!affine) {
+      if (fixed && inst > 1) {
+        const unsigned grid = std::min(blocks, (unsigned)queue_grid<F>());
+        k_msm_accum0_queue<F, true><<<grid, seg_threads<F>(), 0, st>>>(
+            L.srec, total_p, ps, s.k0, L.buckets, ok, L.ppt[1], blocks, L.tileq);
+      } else {
+        const auto kern = fixed ? k_msm_accum0<F, true> : k_msm_accum0<F, false>;
+        kern<<<blocks, seg_threads<F>(), 0, st>>>(L.srec, total_p, ps, s.k0, L.buckets, ok,
+                                                  L.ppt[1]);
+      }
+      ZK_LAUNCHED();
+    }
   }
   for (int l = 1; l < s.levels; l++) {
     const int in = l & 1, out = in ^ 1;

@@ -15,6 +15,9 @@
 //                   thread's work (skewed scalars stay balanced); buckets that
 //                   cross thread ranges leave partial sums that further levels
 //                   of the same kernel combine;
+//                      Large G2 lists first add the runs of a bucket
+//                      pairwise in affine coordinates with shared inversions
+//                      (msm_affine) and accumulate what is left;
 //   5. msm_reduce_l1 / msm_reduce_blk
 //                   sum_b (b+1) S_b per window: running sums over chunks of
 //                   buckets, then block-parallel passes (suffix scan + tree
