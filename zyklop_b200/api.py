@@ -339,7 +339,9 @@ UNIFORM, SKEWED = 0, 1
 
 def table_c_default(log_n):
     """fixed-base window bits used when nothing is tuned for the size"""
-    return min(max(log_n, 8), 20)
+    if log_n <= 13:
+        return max(8, log_n - 2)
+    return 15 if log_n <= 17 else 17 if log_n <= 19 else 20
 
 
 def autotune_msm(group, log_n, dist=UNIFORM, fixed_c=0, ctx=None):

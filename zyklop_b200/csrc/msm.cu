@@ -66,7 +66,7 @@ Shape make_shape(size_t n, bool g2, const MsmConfig& cfg, bool fixed = false, in
   s.records = std::max<size_t>((size_t)s.W * n, 1);
   s.k0 = cfg.k0 > 0 ? cfg.k0 : msm_default_k0(n, fixed);
   s.k1 = cfg.k1;
-  s.chunk = cfg.chunk > 0 ? cfg.chunk : msm_default_chunk(n, fixed, s.c);
+  s.chunk = cfg.chunk > 0 ? cfg.chunk : msm_default_chunk((size_t)s.Wk * s.B, fixed, g2);
   s.J = (s.B + s.chunk - 1) / s.chunk;
   size_t rec = s.records;
   int per_thread = s.k0;
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(seg_threads<F>()) k_msm_accum0_queue(
 // pairwise in affine coordinates before the XYZZ accumulation sees them.  An
 // affine addition costs two Fp2 products, a square and an inversion, and
 // Montgomery's trick over the norms in Fp makes the inversion five Fp products
-// and a norm plus a shared one: about 3000 multiply instructions against 5400
+// and a norm plus a shared one: about 3400 multiply instructions against 6300
 // of the mixed XYZZ addition, with half the live registers (16 warps per SM
 // instead of 8).
 //
@@ -1448,46 +1448,63 @@ MsmResult msm_enqueue(const ScalarSrc& ss, const PointSrc<F>& ps, int inst, size
 
 }  // namespace
 
-// Defaults from autotuner runs (G1 and G2 agree within a few percent):
-// window bits lg - 4 up to 2^16 points, then lg - 3 capped at 16 through
-// 2^22 (a window's 2^15 buckets of XYZZ sums stay L2-resident), growing
-// again by one per doubling beyond 2^22; records per accumulation thread 16
-// up to 2^15 points, 32 up to 2^17, then 64 / 128 (fixed-base, below / from
-// 2^20) or 128 / 256 (windowed, below / from 2^22); buckets per reduction
-// thread 4 up to 2^16 points, 8 up to 2^18, then 16.  Small MSMs are bound
-// by the depth of their dependent additions, so they get short per-thread
-// runs.  Fixed-base sets of 2^19 or more buckets (windows of 20 bits and
-// up) take 32 buckets per reduction thread: timed as whole 2^20 proofs,
-// where four MSMs overlap, k0 128 / chunk 32 ran 23.3 ms against 24.8 ms
-// for 64 / 16 (less reduction work beats a shorter chain there).
-int msm_default_c(size_t n, bool g2) {
-  (void)g2;
+// Defaults, from sweeps of lone MSMs over sizes 2^8 .. 2^22 (tables 2^10 ..
+// 2^20) and of whole 2^13 .. 2^20 proofs.  Small MSMs are bound by the depth
+// of their dependent additions, so they take short per-thread runs, few
+// buckets and short reduction chains; sizes count by the nearest power of two
+// (a circuit's point sets are a little larger than its domain).
+namespace {
+int nearest_log2(size_t n) {
   int lg = 0;
-  while ((size_t(1) << lg) < n) lg++;
-  int c = lg <= 16 ? lg - 4 : std::min(lg - 3, 16 + std::max(0, lg - 22));
-  if (c < 4) c = 4;
-  if (c > 20) c = 20;
-  return c;
+  while (lg < 63 && (size_t(1) << lg) < n) lg++;
+  // below 2^(lg - 1/2): n^2 < 2^(2 lg - 1)
+  if (lg && lg < 32 && n * n < (size_t(1) << (2 * lg - 1))) lg--;
+  return lg;
+}
+}  // namespace
+
+// Window bits: 6 up to 2^10 points (777 points on G1: 0.30 ms, with 4 bits
+// 0.33, with 8 0.31), lg - 5 up to 2^17 (2^16 points: 11 bits 0.74 ms, 12 0.77,
+// 13 0.82), then 15 (2^20 points: 4.33 ms, 16 bits 4.34; a third shorter runs
+// of zero digits on circom-like scalars: 2.08 against 2.17), 16 from 2^22 and
+// one more per doubling beyond.  On G2, whose affine accumulation likes long
+// runs, 11 at 2^17 (2.25 ms, 12 bits 2.42) and 13 at 2^18 (3.47, 15 bits 3.68).
+int msm_default_c(size_t n, bool g2) {
+  const int lg = nearest_log2(n);
+  if (lg <= 17) return std::max(6, g2 && lg == 17 ? lg - 6 : lg - 5);
+  if (g2 && lg == 18) return 13;
+  return lg < 22 ? 15 : std::min(lg - 6, 20);
 }
 
 int msm_effective_c(size_t n, bool g2, const MsmConfig& cfg) {
   return cfg.c > 0 ? cfg.c : msm_default_c(n, g2);
 }
 
+// Sorted records per thread of the XYZZ accumulation: 8 up to 2^13 points
+// (fixed-base 2^12: 0.32 against 0.35 ms with 16), growing to 64 at 2^20
+// (windowed 2^19: 32 2.51 ms, 128 2.96, whose blocks make 1.2 waves), 128 from
+// 2^22 windowed.  Whole 2^20 proofs with tables: 64 19.0 ms, 32 19.4, 128 19.3.
 int msm_default_k0(size_t n, bool fixed) {
-  int lg = 0;
-  while ((size_t(1) << lg) < n) lg++;
+  const int lg = nearest_log2(n);
+  if (lg <= 13) return 8;
   if (lg <= 15) return 16;
-  if (lg <= 17) return 32;
-  if (fixed) return lg <= 19 ? 64 : 128;
-  return lg < 22 ? 128 : 256;
+  if (lg == 18 && !fixed) return 16;
+  if (lg <= 19) return 32;
+  return fixed || lg < 22 ? 64 : 128;
 }
 
-int msm_default_chunk(size_t n, bool fixed, int c) {
-  if (fixed && c >= 20) return 32;
-  int lg = 0;
-  while ((size_t(1) << lg) < n) lg++;
-  return lg <= 16 ? 4 : (lg <= 18 ? 8 : 16);
+// Buckets per lane group of the first reduction level, from the buckets of
+// all sets: enough groups to keep the device busy, then longer chains instead
+// of more groups for the block passes above.  Fixed-base sets (few, large):
+// 8192 groups (G1; 2^17 buckets 16: 1.34 ms, 32 1.39) or 4096 groups of eight
+// lanes (G2); windowed ones ~3100, since every window has a block pass of its
+// own (2^16 points, 24 windows of 2^10: 8 0.74 ms, 16 0.77).
+int msm_default_chunk(size_t buckets, bool fixed, bool g2) {
+  const size_t groups = !fixed ? 3100 : (g2 ? 4096 : 8192);
+  const int most = fixed || buckets > 400000 ? 32 : 16;
+  int chunk = 2;
+  while (chunk < most && groups * chunk < buckets) chunk *= 2;
+  return chunk;
 }
 
 size_t msm_scratch_bytes(size_t n, bool g2, const MsmConfig& cfg) {

@@ -92,7 +92,7 @@ int msm_default_c(size_t n, bool g2);
 // Window bits a windowed MSM of n points runs with under cfg.
 int msm_effective_c(size_t n, bool g2, const MsmConfig& cfg);
 int msm_default_k0(size_t n, bool fixed);
-int msm_default_chunk(size_t n, bool fixed = false, int c = 0);
+int msm_default_chunk(size_t buckets, bool fixed, bool g2);
 
 // Device scratch bytes one MSM of n points needs with this configuration.
 size_t msm_scratch_bytes(size_t n, bool g2, const MsmConfig& cfg);

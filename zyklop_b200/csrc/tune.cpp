@@ -205,8 +205,9 @@ TuneResult autotune_msm(zk_ctx* ctx, int group, int log_n, int dist, int fixed_c
   // a lone MSM favours shorter dependency chains and its timing is noisy.
   double margin = 0;
   if (fixed_c) {
-    cfg.k0 = msm_default_k0(n, true);
-    cfg.chunk = msm_default_chunk(n, true, fixed_c);
+    // (within the candidates below: the shortest runs only suit small sets)
+    cfg.k0 = std::max(16, msm_default_k0(n, true));
+    cfg.chunk = std::max(4, msm_default_chunk(size_t(1) << (fixed_c - 1), true, g2));
     margin = 0.02;
   }
   if (!fixed_c) {
