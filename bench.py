@@ -50,17 +50,26 @@ UNIT = "proofs/s"
 # algorithmic Fp multiplications per MSM point (bucket accumulation with the
 # reference's 16-window, 7M+4S mixed-add decomposition) and IMAD-class ops per
 # Fp multiplication (8x8 limb products lo+hi for a*b and m*p, plus m).  Both
-# are work conventions: the kernels issue 232 IMAD-class ops per Fp product
-# (Karatsuba) and 560 per Fp2 product (two reductions), so a fraction of the
-# carry-chain probe counted this way can exceed the issued one.
+# are work conventions: sums of products share reductions and squares need
+# fewer limb products, so a fraction of the carry-chain probe counted this way
+# can exceed the issued one.
 FP_MULTS_PER_POINT = {"accum_g1": 176.0, "accum_g2": 528.0}
 IMAD_PER_FP_MULT = 264.0
-# what the fixed-base accumulation issues per sorted record (one mixed XYZZ
-# add): G1 6 products x 232 + 2 squares x (72 + 136) + one shared-reduction
-# difference of products (2 x 96 + 136); G2 8 Fp2 products x 560 + 2 Fp2
-# squares x 2 x 232
-ISSUED_IMAD_PER_RECORD = {"accum_g1": 6 * 232 + 2 * (72 + 136) + 2 * 96 + 136,
-                          "accum_g2": 8 * 560 + 2 * 2 * 232}
+# what the fixed-base accumulation issues per sorted record.  A wide product is
+# 128 lo / hi multiply-adds, a wide square 72, a reduction 136.  G1, one mixed
+# XYZZ add: 6 products, 2 squares and a difference of two products with one
+# reduction.  G2, one batched affine add (large lists): a norm, 3 products of
+# the shared inversion and 2 to scale the conjugate, 2 Fp2 products (3 wide
+# products and 2 reductions each) and an Fp2 square (2 products).  Aligned
+# lo / hi pairs run as one wide multiply-add, which the carry-chain probe's
+# unpaired stream does not: issued counts reach 1.05 of it, 0.7 of the nominal
+# 64 multiply-adds per clock and SM.
+ISSUED_IMAD_PER_RECORD = {"accum_g1": 6 * 264 + 2 * (72 + 136) + 2 * 128 + 136,
+                          "accum_g2": (2 * 72 + 136) + 5 * 264 + 2 * (3 * 128 + 2 * 136)
+                          + 2 * 264}
+
+# large G2 lists take the affine rounds and their tail
+ACCUM_KERNEL = {"accum_g1": "k_msm_accum0", "accum_g2": "k_msm_affine + k_msm_affine_tail"}
 
 
 def parse_args():
@@ -312,7 +321,7 @@ def roofline_of(kind, rec, peak, step_ms, records_per_point=None, peak_variants=
         return None
     conv = ku * FP_MULTS_PER_POINT[kind] * IMAD_PER_FP_MULT / (kms / 1e3) / 1e12
     per_point = traffic_per_point().get(kind)
-    r = {"bound": "imad", "kernel": f"k_msm_accum0 ({kind})", "achieved": conv,
+    r = {"bound": "imad", "kernel": f"{ACCUM_KERNEL[kind]} ({kind})", "achieved": conv,
          "peak": peak, "unit": "TIOP/s", "frac": conv / peak, "work": "convention",
          "traffic": per_point * ku / kl if per_point else None,
          "peak_source": "zk_imad_probe (measured carry-chain IMAD throughput)",

@@ -131,11 +131,12 @@ void ProveWs::init() {
   // Stream priorities order block dispatch among a proof's MSM chains when
   // the proof runs alone: the B2 (G2) MSM, the longest chain, first; then
   // stream 0, whose H MSM starts only after the SpMV and the H pipeline; A,
-  // C and B1 fill the SMs left over.  Measured on a 2^20 proof: 22.9 ms
-  // against 23.4 ms with equal priorities (B2 alone first, or the H chain
-  // alone or first, gave less).  Beside other proofs (in-flight batches, the
-  // server) every proof's B2 would outrank the rest of the device's work:
-  // batches ran ~10 % slower, so those workspaces keep equal priorities.
+  // C and B1 fill the SMs left over.  Measured on a 2^20 proof (with G2 on
+  // XYZZ only): 22.9 ms against 23.4 ms with equal priorities (B2 alone
+  // first, or the H chain alone or first, gave less).  Beside other proofs
+  // (in-flight batches, the server) every proof's B2 would outrank the rest
+  // of the device's work: batches ran ~10 % slower, so those workspaces keep
+  // equal priorities.
   int least = 0, greatest = 0;
   ZK_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
   for (int i = 0; i < kStreams; i++) {
