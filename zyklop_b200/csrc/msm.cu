@@ -976,16 +976,8 @@ __global__ void __launch_bounds__(kAffT, kBlocks == 3 ? 3 : 1) k_msm_affine_tail
 // Blocks of the rounds the device holds at once: one wave.
 template <int kBlocks>
 size_t affine_grid_of() {
-  static const int g = [] {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_msm_affine<true, kBlocks>, kAffT,
-                                                      0) != cudaSuccess) {
-      (void)cudaGetLastError();
-      per_sm = 1;
-    }
-    return std::max(1, per_sm) * device_sm_count();
-  }();
-  return (size_t)g;
+  static PerDevice<size_t> known;
+  return resident_blocks(known, k_msm_affine<true, kBlocks>, kAffT, 0);
 }
 size_t affine_grid(int blocks) { return blocks == 3 ? affine_grid_of<3>() : affine_grid_of<4>(); }
 size_t affine_wave(int blocks) { return affine_grid(blocks) * kAffT * kAffMaxSub * kSub; }
@@ -1023,9 +1015,13 @@ void affine_enqueue(const uint2* srec, const uint32_t* total_p, const PointSrc<f
                     size_t records, unsigned char* scratch, xyzz<fp2_t>* buckets, uint32_t* okey,
                     xyzz<fp2_t>* opt, uint32_t ntiles, cudaStream_t st) {
   constexpr size_t smem = kAffT * sizeof(SegNode<fp2_t>);
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_msm_affine_tail<kFixed, kBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  ZK_CUDA(attr);
+  // more than the default 48 KB
+  static PerDevice<bool> allowed;
+  allowed.get(current_device(), [&] {
+    ZK_CUDA(cudaFuncSetAttribute(k_msm_affine_tail<kFixed, kBlocks>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return true;
+  });
   const AffShape shape = aff_shape(aff_span(records, ntiles));
   const uint32_t wave = (uint32_t)affine_grid(kBlocks);
   for (uint32_t t0 = 0; t0 < ntiles; t0 += wave) {
@@ -1303,16 +1299,8 @@ __global__ void __launch_bounds__(128) k_msm_precompute(const F* __restrict__ px
 // Blocks of the persistent level 0 the device holds at once.
 template <class F>
 int queue_grid() {
-  static const int g = [] {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_msm_accum0_queue<F, true>,
-                                                      seg_threads<F>(), 0) != cudaSuccess) {
-      (void)cudaGetLastError();
-      per_sm = 1;
-    }
-    return std::max(1, per_sm) * device_sm_count();
-  }();
-  return g;
+  static PerDevice<size_t> known;
+  return (int)resident_blocks(known, k_msm_accum0_queue<F, true>, seg_threads<F>(), 0);
 }
 
 // The GPU part of one launch chain: a windowed MSM (inst = 1, points from

@@ -702,17 +702,10 @@ __global__ void __launch_bounds__(kPassThreads) k_hpoly_persistent(const __grid_
 #define ZK_HPOLY_PER_SM 4
 #endif
 int hpoly_grid() {
-  static const int g = [] {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hpoly_persistent, kPassThreads,
-                                                      (size_t)8 * 4 * kTile) != cudaSuccess) {
-      (void)cudaGetLastError();
-      per_sm = 1;
-    }
-    per_sm = per_sm < 1 ? 1 : (per_sm > ZK_HPOLY_PER_SM ? ZK_HPOLY_PER_SM : per_sm);
-    return per_sm * device_sm_count();
-  }();
-  return g;
+  static PerDevice<size_t> known;
+  const size_t held = resident_blocks(known, k_hpoly_persistent, kPassThreads, (size_t)8 * 4 * kTile);
+  const int most = ZK_HPOLY_PER_SM * device_sm_count();
+  return held < (size_t)most ? (int)held : most;
 }
 
 }  // namespace

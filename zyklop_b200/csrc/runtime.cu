@@ -226,10 +226,15 @@ void Stager::upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   ZK_CUDA(cudaEventSynchronize(ev[1]));
 }
 
+int current_device() {
+  int dev = 0;
+  ZK_CUDA(cudaGetDevice(&dev));
+  return dev;
+}
+
 int device_sm_count() {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  int n = 0;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, current_device());
   return n;
 }
 

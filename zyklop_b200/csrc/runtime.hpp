@@ -17,6 +17,7 @@
 #include <string>
 
 #include "../../include/zyklop_b200.h"
+#include "per_device.hpp"
 
 namespace zk {
 
@@ -121,6 +122,17 @@ struct Carver {
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-int device_sm_count();
+int current_device();
+int device_sm_count();  // of the current device
+// Blocks of a kernel that the current device holds at once (at least one per
+// SM), looked up once per device.
+template <class Kernel>
+size_t resident_blocks(PerDevice<size_t>& known, Kernel kernel, int threads, size_t smem) {
+  return known.get(current_device(), [&] {
+    int per_sm = 0;
+    ZK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+    return (size_t)(per_sm < 1 ? 1 : per_sm) * device_sm_count();
+  });
+}
 
 }  // namespace zk
