@@ -83,3 +83,32 @@ def test_fixed_base_reduction(api, oracle, points, group, c):
     out, inf = t.run(sc)
     t.close()
     assert not inf and np.array_equal(out, exp)
+
+
+@pytest.mark.parametrize("group", [1, 2])
+def test_empty_buckets_cost_no_products(api, points, group):
+    """15-bit windows over 300 points: nearly all the time of the uniform MSM is
+    the reduction of mostly empty buckets; with zero scalars every addition has
+    an operand at infinity, and a reduction that does its products all the
+    same takes as long"""
+    import time
+    import torch
+    rng = np.random.default_rng(5)
+    px, py, sc = inputs(points, group, 300, "uniform", rng)
+    msm = api.msm_g1 if group == 1 else api.msm_g2
+
+    def best(s):
+        times = []
+        for _ in range(9):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            msm(px, py, s)
+            times.append(time.perf_counter() - t)
+        return min(times)
+    try:
+        api.msm_set_config(group, c=15, chunk=16)
+        full, empty = best(sc), best(np.zeros_like(sc))
+    finally:
+        api.msm_set_config(group)
+    print("uniform %.3f ms, zero %.3f ms" % (1e3 * full, 1e3 * empty))
+    assert empty < 0.5 * full  # 0.30 on G1, 0.17 on G2; 0.70 and 0.65 with the products

@@ -1215,7 +1215,8 @@ __global__ void __launch_bounds__(red_pairs<F>() * quad_lanes<F>()) k_msm_reduce
   if (Jout > 1 || log_span + 1 < depth) {
     lane_t<F> t = zero;
     if (i0 < width) {
-      for (int d = 0; d < log_span; d++) r = quad_dbl(r);
+      if (__any_sync(0xffffffffu, !quad_zero(r, 2)))
+        for (int d = 0; d < log_span; d++) r = quad_dbl(r);
       t = quad_add(r, acc);
     }
     const lane_t<F> s = block_sum<F>(t, sm, width);
