@@ -60,3 +60,11 @@ def test_hpoly_radixes(api, oracle, radix, log_n):
         for bits in (8, 4):
             radix(log_n, bits)
             assert np.array_equal(api.hpoly(a, b, log_n), want), (kind, bits)
+
+
+@pytest.mark.parametrize("log_n", [13, 14, 15])
+def test_hpoly_around_one_wave_of_coset_threads(api, oracle, log_n):
+    """up to 2^13 a thread scales one vector's coefficient, from 2^14 on those of all three"""
+    for kind in ("random", "largest"):
+        a, b = operands(log_n, kind), operands(log_n, kind)[::-1].copy()
+        assert np.array_equal(api.hpoly(a, b, log_n), oracle.hpoly(a, b, log_n)), kind

@@ -382,10 +382,10 @@ __global__ void k_pointwise_mul(const __grid_constant__ HArgs args, size_t n) {
 
 // x[p] *= (1/N) omega_2n^rev(p) for coefficients held in bit-reversed order
 // (the coset shift of src/groth16.cu:914-921 with the INTT scale folded in),
-// for the three vectors of a polynomial at once: the factor is formed once,
+// for kVecs vectors of a polynomial at once: the factor is formed once,
 // and 1/N is an exact shift.  Results stay below 2r for the DIT passes.
-template <bool CG>
-__device__ __forceinline__ void coset_elem(fr_t* const (&v)[3], size_t p,
+template <bool CG, int kVecs>
+__device__ __forceinline__ void coset_elem(fr_t* (&v)[kVecs], size_t p,
                                            const fr_t* __restrict__ tw, int tw_shift, int L,
                                            const fr_t& w2n) {
   const size_t e = rev_bits(p, L);
@@ -399,17 +399,20 @@ __device__ __forceinline__ void coset_elem(fr_t* const (&v)[3], size_t p,
   }
   if (e & 1) t = t * w2n;  // the upper half of the positions
 #pragma unroll
-  for (int q = 0; q < 3; q++)
+  for (int q = 0; q < kVecs; q++)
     fe_store(v[q], p, fr_div_pow2(fr_mul_lazy(fr_load<CG>(v[q], p), t), L));
 }
 
+template <int kVecs>
 __global__ void k_coset_scale(PassArgs args, const fr_t* __restrict__ tw, int tw_shift, int L,
                               fr_t w2n) {
   const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >> L) return;
-  const int j = 3 * blockIdx.y;
-  fr_t* const v[3] = {args.in[j], args.in[j + 1], args.in[j + 2]};
-  coset_elem<false>(v, p, tw, tw_shift, L, w2n);
+  const int j = kVecs * blockIdx.y;
+  fr_t* v[kVecs];
+#pragma unroll
+  for (int q = 0; q < kVecs; q++) v[q] = args.in[j + q];
+  coset_elem<false, kVecs>(v, p, tw, tw_shift, L, w2n);
 }
 
 // h = A*B - C, decoded to canonical (src/groth16.cu:935-948, 218-226), per
@@ -462,6 +465,11 @@ void run_pass(bool dit, const PassArgs& args, int count, const fr_t* tw, int tw_
   while ((1 << (log_g + 1 + k)) <= kTile && (size_t(1) << (log_g + 1)) <= groups &&
          (lo == 0 || log_g + 1 <= lo))
     log_g++;
+  // A launch that leaves half of the SMs idle is bound by one block's latency:
+  // smaller tiles, down to one element a thread to load and store (H pipeline
+  // at 2^9 / 2^12: 77 / 78 us, with full tiles 85 / 88).
+  const size_t sms = (size_t)device_sm_count();
+  while (log_g && (1 << (k + log_g)) > kPassThreads && 2 * count * (groups >> log_g) <= sms) log_g--;
   const size_t blocks = groups >> log_g;
   const size_t smem = (size_t)8 * 4 * (size_t(1) << (k + log_g));
   dim3 grid((unsigned)blocks, count);
@@ -575,8 +583,16 @@ void hpoly_batch(NttTables& tw, int count, uint64_t* const* aw, uint64_t* const*
   k_pointwise_mul<<<dim3(blocks_for(n), count), 256, 0, st>>>(ha, n);
   ZK_LAUNCHED();
   dif(abc, abc, abc, 3 * count, tw.inv.as<fr_t>(), shift, log_n, tw.pass_bits[log_n], st);
-  k_coset_scale<<<dim3(blocks_for(n), count), kElemThreads, 0, st>>>(
-      abc, tw.fwd.as<fr_t>(), shift, log_n, to_dev(host_root(log_n + 1)));
+  // One thread per element and vector while these do not fill the device
+  // (2^8 / 2^13: 62 / 80 us, with three vectors a thread 66 / 82), then one per
+  // element (2^17 / 2^20: 252.5 / 1459 us against 254.5 / 1480).
+  const fr_t w2n = to_dev(host_root(log_n + 1));
+  if (3 * count * n <= (size_t)device_sm_count() * 256)
+    k_coset_scale<1><<<dim3(blocks_for(n), 3 * count), kElemThreads, 0, st>>>(
+        abc, tw.fwd.as<fr_t>(), shift, log_n, w2n);
+  else
+    k_coset_scale<3><<<dim3(blocks_for(n), count), kElemThreads, 0, st>>>(
+        abc, tw.fwd.as<fr_t>(), shift, log_n, w2n);
   ZK_LAUNCHED();
   dit(abc, 3 * count, tw.fwd.as<fr_t>(), shift, log_n, tw.pass_bits[log_n], st);
   k_h_final<<<dim3(blocks_for(n), count), 256, 0, st>>>(ha, n);
@@ -675,9 +691,9 @@ __global__ void __launch_bounds__(kPassThreads) k_hpoly_persistent(const __grid_
       pass_tile<false, true>(x, x, local % nb, p.tw_inv, J.shift, J.L, J.lo[pi], J.k[pi],
                              J.log_g[pi], sm);
     } else if (st == np + 1) {
-      fr_t* const v[3] = {J.a, J.b, J.c};
+      fr_t* v[3] = {J.a, J.b, J.c};
       const size_t i = (size_t)local * kPassThreads + threadIdx.x;
-      if (i < n) coset_elem<true>(v, i, p.tw_fwd, J.shift, J.L, J.w2n);
+      if (i < n) coset_elem<true, 3>(v, i, p.tw_fwd, J.shift, J.L, J.w2n);
     } else if (st <= 2 * np + 1) {
       const uint32_t pi = st - np - 2, nb = J.pass_blocks[pi];
       const uint32_t arr = local / nb;
