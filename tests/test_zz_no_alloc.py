@@ -124,3 +124,43 @@ def test_noalloc_refuses_a_capturing_stream(api):
         g.capture_end()
     assert rc == 9  # ZK_ENOTSUP
     assert b"captur" in lib().zk_last_error()
+
+
+def test_noalloc_layout_fits_the_array_for_every_size(api):
+    from zyklop_b200._lib import check, lib
+    need = ctypes.c_size_t(0)
+    most = 0
+    for n in range(MAX_POINTS + 1):
+        check(lib().zk_msm_scratch_bytes(None, 1, n, ctypes.byref(need)))
+        most = max(most, need.value)
+    print("largest layout %.2f MiB" % (most / 2**20))
+    assert most <= 24 << 20
+
+
+@pytest.mark.parametrize("n", [100, 4000])
+def test_noalloc_takes_the_settings_of_its_size(api, n):
+    """the same kernels with the same settings take about the same time; runs and
+    chains of the largest size took more than twice as long"""
+    import time
+    import torch
+    from zyklop_b200._lib import check, lib
+    rng = np.random.default_rng(n)
+    px, py = api.mul_generator(1, scalars(rng, n))
+    dx, dy, ds = (api.to_device(a) for a in (px, py, scalars(rng, n)))
+    out = np.zeros(8, np.uint64)
+
+    def plain():
+        check(lib().zk_msm_g1(None, api.ptr(dx), api.ptr(dy), api.ptr(ds), n,
+                              out.ctypes.data_as(ctypes.POINTER(ctypes.c_uint64)), None))
+
+    def best(f):
+        times = []
+        for _ in range(15):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            f()
+            times.append(time.perf_counter() - t)
+        return min(times)
+    a, b = best(lambda: noalloc(api, dx, dy, ds, n)), best(plain)
+    print("noalloc %.3f ms, zk_msm_g1 %.3f ms" % (1e3 * a, 1e3 * b))
+    assert a < 1.5 * b

@@ -114,10 +114,9 @@ extern "C" int zk_msm_g1_noalloc(const uint64_t* d_px, const uint64_t* d_py,
     ~ProfilerOff() { zk::set_current_profiler(saved); }
   } profiler_off;
   ZK_API_BEGIN
-  // fixed settings: the 24 MiB bound above is checked against this layout
-  zk::MsmConfig cfg;
-  cfg.k0 = 64;
-  cfg.chunk = 16;
+  // the settings zk_msm_g1 takes by size: the largest layout up to 2^16 points
+  // is 16.05 MiB (its test asks for every n)
+  const zk::MsmConfig cfg;
   ZK_REQUIRE(zk::msm_scratch_bytes(n, false, cfg) <= kNoAllocScratchBytes, ZK_EINTERNAL,
              "zk_msm_g1_noalloc: scratch layout exceeds the fixed array");
   const zk::MsmResult r = zk::msm_g1_enqueue(zk::points_soa(d_px, d_py), d_scalars, n, scratch,
