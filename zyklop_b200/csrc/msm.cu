@@ -7,6 +7,7 @@
 #include <cstring>
 #include <vector>
 
+#include "affine_layout.hpp"
 #include "curve_quad.cuh"
 #include "host_field.hpp"
 #include "msm.hpp"
@@ -531,54 +532,16 @@ __global__ void __launch_bounds__(seg_threads<F>()) k_msm_accum0_queue(
 // of `ends` is set when point j is the last of its run.  A round about halves
 // the points, and the slots are sized for that; a block with runs too short
 // for it (or for one round to pay) skips the rounds.
-constexpr int kAffT = 128;      // threads per block
-constexpr int kSub = 64;        // points per sub-segment
-constexpr int kAffMaxSub = 3;   // sub-segments per thread: S <= 192
-constexpr int kAffMinS = 32;    // records per thread, at least
 constexpr int kAffLeast = 8;    // additions left per thread for a round to pay
 constexpr uint32_t kAffUntouched = 1u << 31;  // state: points still the table's
 constexpr uint32_t kAffFirst = 1u << 30;      // state: points in slot buffer 1
-
-// Layout of one resident block's scratch, interleaved by thread, for at most
-// S records per thread.
-struct AffShape {
-  int nsub;       // sub-segments per thread
-  int slots[2];   // slots per sub-segment: buffer 1 takes the first round's
-                  // results, buffer 0 the second's, and so on in turn
-  uint32_t pre;   // byte offsets of the pairs' prefixes and norms,
-  uint32_t mask;  // of the masks
-  uint32_t state; // and of the final state
-  uint32_t bytes;
-};
-__host__ __device__ inline AffShape aff_shape(int S) {
-  AffShape a;
-  a.nsub = (S + kSub - 1) / kSub;
-  const int sub = S < kSub ? S : kSub;
-  a.slots[0] = sub / 2;
-  a.slots[1] = sub - sub / 4;
-  const uint32_t buf = (uint32_t)(a.nsub * kAffT) * 2 * sizeof(fp2_t);
-  a.pre = buf * (a.slots[0] + a.slots[1]);
-  a.mask = a.pre + (uint32_t)(a.nsub * (sub / 2) * kAffT) * 2 * sizeof(fp_t);
-  a.state = a.mask + (uint32_t)(a.nsub * 3 * kAffT) * sizeof(uint64_t);
-  a.bytes = a.state + kAffT * sizeof(uint32_t);
-  return a;
-}
-static_assert(kAffMaxSub * kSub < 256 && kAffMinS % 4 == 0, "layout of the affine scratch");
-
-// Records per thread (even) of a list of `total` over ntiles tiles: spread
-// evenly by the actual number, so skewed scalars, whose zero digits make no
-// records, leave no tile idle.
-__host__ __device__ inline int aff_span(size_t total, uint32_t ntiles) {
-  const size_t lanes = (size_t)ntiles * kAffT;
-  const int S = ((int)((total + lanes - 1) / lanes) + 1) & ~1;
-  return S < kAffMinS ? kAffMinS : S;
-}
+static_assert(sizeof(fp2_t) * 2 == kAffPoint && sizeof(fp_t) * 2 == kAffPair, "affine_layout.hpp");
 
 struct AffScratch {
   unsigned char* base;
   const AffShape& a;
   __device__ __forceinline__ fp2_t* slot(int buf, int h, int j) const {
-    const int row = h * a.slots[buf] + j + (buf ? a.nsub * a.slots[0] : 0);
+    const int row = h * a.slots[buf] + j + (buf ? a.rows : 0);
     return reinterpret_cast<fp2_t*>(base) + 2 * (uint32_t)(row * kAffT + threadIdx.x);
   }
   // prefix product and norm of pair k
@@ -749,7 +712,7 @@ __global__ void __launch_bounds__(kAffT, kBlocks) k_msm_affine(
     links += __popcll(C);
     const int o1 = cnt - __popcll(M);
     const int o2 = o1 - __popcll(aff_pairs(aff_links(aff_squeeze(ends, M), o1)));
-    fits = fits && o1 <= shape.slots[1] && o2 <= shape.slots[0];
+    fits = fits && o1 <= shape.limit(h, 1) && o2 <= shape.limit(h, 0);
   }
   const int lanes = __syncthreads_count(len > 0);
 
