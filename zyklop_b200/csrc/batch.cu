@@ -105,17 +105,20 @@ void fused_launch(zk_ctx* ctx, FusedWs& f, Group& g, const uint64_t* const* wits
   const zk_circuit* c0 = g.jobs[0].c;
   const MsmConfig cfgw = msm_config_for(ctx, false, nmaxw, c0->dist, c1);
   const MsmConfig cfgh = msm_config_for(ctx, false, nmaxh, kDistUniform, c1);
-  const MsmConfig cfg2 = msm_config_for(ctx, true, nmaxw, c0->dist, c2);
+  MsmConfig cfg2 = msm_config_for(ctx, true, nmaxw, c0->dist, c2);
   const int instw = (int)nj * g.per_job, insth = (int)nj, inst2 = (int)nj;
   f.we.ensure(wbytes);
   f.poly.ensure(pbytes);
   f.g1w.ensure(msm_scratch_bytes_fixed(nw, false, c1, cfgw, instw));
   f.gh.ensure(msm_scratch_bytes_fixed(nh, false, c1, cfgh, insth));
-  f.g2.ensure(msm_scratch_bytes_fixed(n2, true, c2, cfg2, inst2));
   f.win1w.ensure((size_t)instw * 2 * 128);
   f.winh.ensure((size_t)insth * 2 * 128);
   f.win2.ensure((size_t)inst2 * 2 * 256);
   ctx->ntt.ensure(log_max, f.s1);
+  // last, with what the other buffers leave
+  msm_ensure_scratch(f.g2, cfg2, [&](const MsmConfig& k) {
+    return msm_scratch_bytes_fixed(n2, true, c2, k, inst2);
+  });
 
   // stage the witnesses (after earlier work on the context stream)
   ZK_CUDA(cudaStreamWaitEvent(f.s1, ev_begin, 0));
@@ -153,8 +156,8 @@ void fused_launch(zk_ctx* ctx, FusedWs& f, Group& g, const uint64_t* const* wits
       key.push_back(j.c->id);
       key.push_back((uint64_t)ctx->ntt.pass_bits[j.c->log_n]);
     }
-    for (const MsmConfig* m : {&cfgw, &cfgh, &cfg2})
-      for (int v : {m->c, m->k0, m->k1, m->chunk}) key.push_back((uint64_t)(int64_t)v);
+    for (const MsmConfig* m : {&cfgw, &cfgh, (const MsmConfig*)&cfg2})
+      for (int v : {m->c, m->k0, m->k1, m->chunk, (int)m->affine}) key.push_back((uint64_t)(int64_t)v);
     for (const void* q : {f.we.ptr, f.poly.ptr, f.g1w.ptr, f.gh.ptr, f.g2.ptr, f.win1w.ptr,
                           f.winh.ptr, f.win2.ptr, f.hsync.ptr, f.hflag.ptr})
       key.push_back((uint64_t)(uintptr_t)q);

@@ -211,8 +211,10 @@ int zk_ntt(zk_ctx* ctx, uint64_t* d_a, uint32_t log_n, int inverse) {
   std::lock_guard<std::mutex> g(ctx->mu);
   ZK_REQUIRE(d_a, ZK_EINVAL, "zk_ntt: NULL buffer");
   ZK_REQUIRE(log_n <= (uint32_t)kMaxLogN, ZK_EINVAL, "zk_ntt: log_n > 27");
-  ctx->ntt_scratch.ensure((size_t)32 << log_n);
-  ntt_inplace(ctx->ntt, d_a, (int)log_n, inverse != 0, ctx->ntt_scratch.ptr, ctx->stream);
+  with_room(ctx, [&] {  // memory runs out before the first pass
+    ctx->ntt_scratch.ensure((size_t)32 << log_n);
+    ntt_inplace(ctx->ntt, d_a, (int)log_n, inverse != 0, ctx->ntt_scratch.ptr, ctx->stream);
+  });
   ZK_CUDA(cudaStreamSynchronize(ctx->stream));
   ZK_API_END
 }
@@ -223,8 +225,10 @@ int zk_hpoly(zk_ctx* ctx, uint64_t* d_aw, uint64_t* d_bw, uint32_t log_n, uint64
   std::lock_guard<std::mutex> g(ctx->mu);
   ZK_REQUIRE(d_aw && d_bw && d_h, ZK_EINVAL, "zk_hpoly: NULL buffer");
   ZK_REQUIRE(log_n >= 1 && log_n < (uint32_t)kMaxLogN, ZK_EINVAL, "zk_hpoly: log_n out of range");
-  ctx->ntt_scratch.ensure((size_t)32 << log_n);
-  hpoly(ctx->ntt, d_aw, d_bw, ctx->ntt_scratch.as<uint64_t>(), (int)log_n, d_h, ctx->stream);
+  with_room(ctx, [&] {
+    ctx->ntt_scratch.ensure((size_t)32 << log_n);
+    hpoly(ctx->ntt, d_aw, d_bw, ctx->ntt_scratch.as<uint64_t>(), (int)log_n, d_h, ctx->stream);
+  });
   ZK_CUDA(cudaStreamSynchronize(ctx->stream));
   ZK_API_END
 }
@@ -236,8 +240,11 @@ int zk_msm_g1(zk_ctx* ctx, const uint64_t* d_px, const uint64_t* d_py, const uin
   std::lock_guard<std::mutex> g(ctx->mu);
   ZK_REQUIRE(h_out, ZK_EINVAL, "zk_msm_g1: NULL output");
   ZK_REQUIRE(n == 0 || (d_px && d_py && d_scalars), ZK_EINVAL, "zk_msm_g1: NULL input");
-  const bool inf = msm_g1_run(points_soa(d_px, d_py), d_scalars, n, ctx->msm_scratch,
-                              msm_config_for(ctx, false, n, ctx->scalar_dist, 0), ctx->stream, h_out);
+  bool inf = false;
+  with_room(ctx, [&] {
+    inf = msm_g1_run(points_soa(d_px, d_py), d_scalars, n, ctx->msm_scratch,
+                     msm_config_for(ctx, false, n, ctx->scalar_dist, 0), ctx->stream, h_out);
+  });
   if (is_inf) *is_inf = inf ? 1 : 0;
   ZK_API_END
 }
@@ -249,8 +256,11 @@ int zk_msm_g2(zk_ctx* ctx, const uint64_t* d_px, const uint64_t* d_py, const uin
   std::lock_guard<std::mutex> g(ctx->mu);
   ZK_REQUIRE(h_out, ZK_EINVAL, "zk_msm_g2: NULL output");
   ZK_REQUIRE(n == 0 || (d_px && d_py && d_scalars), ZK_EINVAL, "zk_msm_g2: NULL input");
-  const bool inf = msm_g2_run(points_soa(d_px, d_py), d_scalars, n, ctx->msm_scratch,
-                              msm_config_for(ctx, true, n, ctx->scalar_dist, 0), ctx->stream, h_out);
+  bool inf = false;
+  with_room(ctx, [&] {
+    inf = msm_g2_run(points_soa(d_px, d_py), d_scalars, n, ctx->msm_scratch,
+                     msm_config_for(ctx, true, n, ctx->scalar_dist, 0), ctx->stream, h_out);
+  });
   if (is_inf) *is_inf = inf ? 1 : 0;
   ZK_API_END
 }

@@ -22,7 +22,7 @@ int zk_circuit_load_file(zk_ctx* ctx, const char* zkey_path, zk_circuit** out) {
   ctx = resolve_ctx(ctx);
   std::lock_guard<std::mutex> g(ctx->mu);
   auto f = BinFile::open(zkey_path, "zkey", 1);
-  *out = circuit_load(ctx, *f);
+  with_room(ctx, [&] { *out = circuit_load(ctx, *f); });
   ZK_API_END
 }
 
@@ -33,7 +33,7 @@ int zk_circuit_load_mem(zk_ctx* ctx, const uint8_t* zkey, size_t len, zk_circuit
   ctx = resolve_ctx(ctx);
   std::lock_guard<std::mutex> g(ctx->mu);
   auto f = BinFile::wrap(zkey, len, "zkey", 1);
-  *out = circuit_load(ctx, *f);
+  with_room(ctx, [&] { *out = circuit_load(ctx, *f); });
   ZK_API_END
 }
 
@@ -61,7 +61,7 @@ int zk_circuit_precompute(zk_circuit* c, int c_g1, int c_g2) {
   ZK_REQUIRE(c, ZK_EINVAL, "zk_circuit_precompute: NULL circuit");
   enter_ctx(c->ctx);
   std::lock_guard<std::mutex> g(c->ctx->mu);
-  circuit_precompute(c, c_g1, c_g2);
+  with_room(c->ctx, [&] { circuit_precompute(c, c_g1, c_g2); });
   ZK_API_END
 }
 
@@ -81,7 +81,7 @@ int zk_msm_table_create(zk_ctx* ctx, int group, const uint64_t* d_px, const uint
   t->n = n;
   t->c = c ? c : table_c_for(ctx, group == 2, n, ctx->scalar_dist);
   ZK_REQUIRE(t->c >= 4 && t->c <= 22, ZK_EINVAL, "zk_msm_table_create: c must be 0 or 4..22");
-  t->table.ensure(msm_table_bytes(n ? n : 1, group == 2, t->c));
+  with_room(ctx, [&] { t->table.ensure(msm_table_bytes(n ? n : 1, group == 2, t->c)); });
   msm_precompute(group == 2, points_soa(d_px, d_py), n, t->c, t->table.ptr, ctx->stream);
   ZK_CUDA(cudaStreamSynchronize(ctx->stream));
   *out = t.release();
@@ -96,27 +96,32 @@ int zk_msm_table_run(zk_msm_table* t, const uint64_t* d_scalars, size_t n, uint6
   ZK_REQUIRE(n == 0 || d_scalars, ZK_EINVAL, "zk_msm_table_run: NULL scalars");
   zk_ctx* ctx = enter_ctx(t->ctx);
   std::lock_guard<std::mutex> g(ctx->mu);
-  const bool g2 = t->group == 2;
-  const MsmConfig cfg = msm_config_for(ctx, g2, t->n, ctx->scalar_dist, t->c);
-  // the table's records are laid out for t->n points: run over all of them
-  // with zero scalars past n (a prefix of the table is not a table)
-  const size_t cnt = t->n;
-  DeviceBuffer sc;
-  const uint64_t* scal = d_scalars;
-  if (n < cnt) {
-    sc.ensure(32 * cnt);
-    ZK_CUDA(cudaMemsetAsync(sc.ptr, 0, 32 * cnt, ctx->stream));
-    if (n) ZK_CUDA(cudaMemcpyAsync(sc.ptr, d_scalars, 32 * n, cudaMemcpyDeviceToDevice, ctx->stream));
-    scal = sc.as<uint64_t>();
-  }
-  ctx->msm_scratch.ensure(msm_scratch_bytes_fixed(cnt, g2, t->c, cfg));
-  const MsmResult r = msm_enqueue_fixed(g2, t->table.ptr, scal, cnt, t->c, ctx->msm_scratch.ptr,
-                                        ctx->msm_scratch.cap, cfg, ctx->stream);
-  alignas(16) uint8_t h[1024];
-  ZK_REQUIRE(r.bytes <= sizeof(h), ZK_EINTERNAL, "zk_msm_table_run: result too large");
-  ZK_CUDA(cudaMemcpyAsync(h, r.d_data, r.bytes, cudaMemcpyDeviceToHost, ctx->stream));
-  ZK_CUDA(cudaStreamSynchronize(ctx->stream));
-  const bool inf = g2 ? msm_g2_combine(h, r, h_out) : msm_g1_combine(h, r, h_out);
+  bool inf = false;
+  with_room(ctx, [&] {
+    const bool g2 = t->group == 2;
+    MsmConfig cfg = msm_config_for(ctx, g2, t->n, ctx->scalar_dist, t->c);
+    // the table's records are laid out for t->n points: run over all of them
+    // with zero scalars past n (a prefix of the table is not a table)
+    const size_t cnt = t->n;
+    DeviceBuffer sc;
+    const uint64_t* scal = d_scalars;
+    if (n < cnt) {
+      sc.ensure(32 * cnt);
+      ZK_CUDA(cudaMemsetAsync(sc.ptr, 0, 32 * cnt, ctx->stream));
+      if (n) ZK_CUDA(cudaMemcpyAsync(sc.ptr, d_scalars, 32 * n, cudaMemcpyDeviceToDevice, ctx->stream));
+      scal = sc.as<uint64_t>();
+    }
+    msm_ensure_scratch(ctx->msm_scratch, cfg, [&](const MsmConfig& k) {
+      return msm_scratch_bytes_fixed(cnt, g2, t->c, k);
+    });
+    const MsmResult r = msm_enqueue_fixed(g2, t->table.ptr, scal, cnt, t->c, ctx->msm_scratch.ptr,
+                                          ctx->msm_scratch.cap, cfg, ctx->stream);
+    alignas(16) uint8_t h[1024];
+    ZK_REQUIRE(r.bytes <= sizeof(h), ZK_EINTERNAL, "zk_msm_table_run: result too large");
+    ZK_CUDA(cudaMemcpyAsync(h, r.d_data, r.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    ZK_CUDA(cudaStreamSynchronize(ctx->stream));
+    inf = g2 ? msm_g2_combine(h, r, h_out) : msm_g1_combine(h, r, h_out);
+  });
   if (is_inf) *is_inf = inf ? 1 : 0;
   ZK_API_END
 }
@@ -137,7 +142,7 @@ int zk_prove(zk_circuit* c, const uint64_t* h_witness, size_t n_witness, const u
   ZK_REQUIRE((r == nullptr) == (s == nullptr), ZK_EINVAL, "zk_prove: give both r and s or neither");
   enter_ctx(c->ctx);
   std::lock_guard<std::mutex> g(c->ctx->mu);
-  prove(c, h_witness, n_witness, false, r, s, proof, nullptr);
+  with_room(c->ctx, [&] { prove(c, h_witness, n_witness, false, r, s, proof, nullptr); });
   ZK_API_END
 }
 
@@ -149,7 +154,7 @@ int zk_prove_device(zk_circuit* c, const uint64_t* d_witness, size_t n_witness, 
              "zk_prove_device: give both r and s or neither");
   enter_ctx(c->ctx);
   std::lock_guard<std::mutex> g(c->ctx->mu);
-  prove(c, d_witness, n_witness, true, r, s, proof, nullptr);
+  with_room(c->ctx, [&] { prove(c, d_witness, n_witness, true, r, s, proof, nullptr); });
   ZK_API_END
 }
 
@@ -163,7 +168,7 @@ int zk_prove_intermediates(zk_circuit* c, const uint64_t* h_witness, size_t n_wi
   dbg.aw = aw;
   dbg.bw = bw;
   dbg.h = h;
-  prove(c, h_witness, n_witness, false, nullptr, nullptr, proof, &dbg);
+  with_room(c->ctx, [&] { prove(c, h_witness, n_witness, false, nullptr, nullptr, proof, &dbg); });
   ZK_API_END
 }
 
@@ -180,7 +185,7 @@ int zk_prove_traced(zk_circuit* c, const uint64_t* h_witness, size_t n_witness,
   dbg.eb = trace->eb;
   dbg.ec = trace->ec;
   dbg.h = trace->h;
-  prove(c, h_witness, n_witness, false, nullptr, nullptr, proof, &dbg);
+  with_room(c->ctx, [&] { prove(c, h_witness, n_witness, false, nullptr, nullptr, proof, &dbg); });
   memcpy(trace->msm_a, dbg.msm_a, sizeof dbg.msm_a);
   memcpy(trace->msm_b2, dbg.msm_b2, sizeof dbg.msm_b2);
   memcpy(trace->msm_c, dbg.msm_c, sizeof dbg.msm_c);
@@ -201,11 +206,14 @@ int zk_prove_batch(zk_ctx* ctx, size_t count, zk_circuit* const* circuits,
     fused = count > 0 && circuits;
     for (size_t i = 0; fused && i < count; i++) fused = circuits[i] && circuits[i]->tab_c[0] != 0;
   }
-  if (fused)
-    prove_batch_fused(ctx, count, circuits, witnesses, n_witness, on_device != 0, r, s, proofs,
-                      ctx->batch_group);
-  else
-    prove_batch(ctx, count, circuits, witnesses, n_witness, on_device != 0, r, s, proofs, inflight);
+  with_room(ctx, [&] {
+    if (fused)
+      prove_batch_fused(ctx, count, circuits, witnesses, n_witness, on_device != 0, r, s, proofs,
+                        ctx->batch_group);
+    else
+      prove_batch(ctx, count, circuits, witnesses, n_witness, on_device != 0, r, s, proofs,
+                  inflight);
+  });
   ZK_API_END
 }
 
@@ -246,7 +254,7 @@ int zk_groth16_prove_mem(zk_ctx* ctx, const uint8_t* zkey, size_t zkey_len, cons
   auto zf = BinFile::wrap(zkey, zkey_len, "zkey", 1);
   auto wf = BinFile::wrap(wtns, wtns_len, "wtns", 2);
   const WtnsView w = parse_wtns(*wf);
-  prove_oneshot(ctx, *zf, w.values, w.n_vars, proof);
+  with_room(ctx, [&] { prove_oneshot(ctx, *zf, w.values, w.n_vars, proof); });
   ZK_API_END
 }
 
@@ -259,7 +267,7 @@ int zk_groth16_prove_files(zk_ctx* ctx, const char* zkey_path, const char* wtns_
   auto zf = BinFile::open(zkey_path, "zkey", 1);
   auto wf = BinFile::open(wtns_path, "wtns", 2);
   const WtnsView w = parse_wtns(*wf);
-  prove_oneshot(ctx, *zf, w.values, w.n_vars, proof);
+  with_room(ctx, [&] { prove_oneshot(ctx, *zf, w.values, w.n_vars, proof); });
   ZK_API_END
 }
 

@@ -39,4 +39,26 @@ inline zk_ctx* enter_ctx(zk_ctx* ctx) {
 
 // ctx or the per-device default context, entered
 inline zk_ctx* resolve_ctx(zk_ctx* ctx) { return enter_ctx(ctx ? ctx : default_ctx()); }
+
+// Runs a call (under ctx's lock).  One that runs out of device memory runs once
+// more without the affine G2 accumulation, after ctx's idle workspaces gave
+// back their G2 arenas: scratch that is there for speed makes no call fail.
+template <class Call>
+void with_room(zk_ctx* ctx, Call call) {
+  try {
+    call();
+    return;
+  } catch (const Error& e) {
+    if (e.code != ZK_ENOMEM) throw;
+  }
+  struct WithoutAffine {
+    zk_ctx* c;
+    explicit WithoutAffine(zk_ctx* c) : c(c) {
+      drop_g2_scratch(c);
+      c->affine = false;
+    }
+    ~WithoutAffine() { c->affine = true; }
+  } without(ctx);
+  call();
+}
 }  // namespace zk

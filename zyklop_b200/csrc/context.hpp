@@ -58,6 +58,7 @@ struct ProveWs {
   std::vector<Graph> graphs;
   void init();
   void drop_graph();
+  void drop_g2_scratch();  // of an idle workspace
   cudaEvent_t ev_begin_pool() { init(); return ev_begin; }
   ~ProveWs();
 };
@@ -103,6 +104,7 @@ struct zk_ctx {
   zk::DeviceBuffer msm_scratch;
   zk::MsmConfig msm_cfg[2];       // explicit settings (c != 0) or defaults
   zk::TuneTable tune;             // autotuned settings
+  bool affine = true;             // off while a call runs again for want of memory
   int scalar_dist = 0;            // distribution hint for zk_msm_g1 / g2
   zk::ProveWs ws{true};  // single proofs (ordered streams)
   std::vector<std::unique_ptr<zk::ProveWs>> pool;  // in-flight batch workspaces
@@ -122,6 +124,8 @@ namespace zk {
 
 // Per-device default context (created on first use).
 zk_ctx* default_ctx();
+// Releases the G2 arenas of ctx's workspaces, idle between calls.
+void drop_g2_scratch(zk_ctx* ctx);
 // Makes ctx's device current for the calling thread.
 void use_device(zk_ctx* ctx);
 

@@ -72,7 +72,7 @@ Shape make_shape(size_t n, bool g2, const MsmConfig& cfg, bool fixed = false, in
   size_t rec = s.records;
   int per_thread = s.k0;
   s.levels = 0;
-  s.affine = g2 ? affine_tiles(s.records, (size_t)s.Wk * s.B) : 0;
+  s.affine = g2 && cfg.affine ? affine_tiles(s.records, (size_t)s.Wk * s.B) : 0;
   if (s.affine) {
     s.lvl_records[0] = rec;
     s.lvl_blocks[0] = s.affine;
@@ -1670,8 +1670,9 @@ bool msm_g1_run(const PointsView& pts, const uint64_t* scalars, size_t n, Device
 }
 
 bool msm_g2_run(const PointsView& pts, const uint64_t* scalars, size_t n, DeviceBuffer& scratch,
-                const MsmConfig& cfg, cudaStream_t st, uint64_t out[16]) {
-  scratch.ensure(msm_scratch_bytes(n, true, cfg));
+                MsmConfig cfg, cudaStream_t st, uint64_t out[16]) {
+  msm_ensure_scratch(scratch, cfg,
+                     [&](const MsmConfig& k) { return msm_scratch_bytes(n, true, k); });
   const MsmResult r = msm_g2_enqueue(pts, scalars, n, scratch.ptr, scratch.cap, cfg, st);
   std::vector<uint8_t> h(r.bytes);
   ZK_CUDA(cudaMemcpyAsync(h.data(), r.d_data, r.bytes, cudaMemcpyDeviceToHost, st));

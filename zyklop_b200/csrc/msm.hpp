@@ -42,10 +42,22 @@ struct MsmConfig {
                       // (0 = choose from n)
   int k1 = 16;        // partial records per thread in later levels
   int chunk = 0;      // buckets per thread in the bucket reduction (0 = choose from n)
+  bool affine = true; // large G2 lists: the batched affine accumulation, whose scratch
+                      // is several times the rest of the arena
   bool operator==(const MsmConfig& o) const {
-    return c == o.c && k0 == o.k0 && k1 == o.k1 && chunk == o.chunk;
+    return c == o.c && k0 == o.k0 && k1 == o.k1 && chunk == o.chunk && affine == o.affine;
   }
 };
+
+// Sizes a G2 MSM's arena to bytes_of(cfg).  Where the device has no room for
+// the affine accumulation's scratch, cfg gives that up: the MSM is slower and
+// its result the same.
+template <class Bytes>
+void msm_ensure_scratch(DeviceBuffer& scratch, MsmConfig& cfg, Bytes bytes_of) {
+  if (cfg.affine && scratch.try_ensure(bytes_of(cfg))) return;
+  cfg.affine = false;
+  scratch.ensure(bytes_of(cfg));
+}
 
 // Affine input points: x of point i at x + i*stride coordinates, y likewise.
 // stride 1 = separate x / y arrays (the reference's SoA msm_g1 arguments);
@@ -149,6 +161,6 @@ bool msm_g2_combine_inst(const void* h_data, const MsmResult& r, int inst, uint6
 bool msm_g1_run(const PointsView& pts, const uint64_t* scalars, size_t n, DeviceBuffer& scratch,
                 const MsmConfig& cfg, cudaStream_t stream, uint64_t out[8]);
 bool msm_g2_run(const PointsView& pts, const uint64_t* scalars, size_t n, DeviceBuffer& scratch,
-                const MsmConfig& cfg, cudaStream_t stream, uint64_t out[16]);
+                MsmConfig cfg, cudaStream_t stream, uint64_t out[16]);
 
 }  // namespace zk

@@ -357,8 +357,30 @@ void ws_scratch_needs(zk_circuit* c, bool blind, const MsmConfig cfg[ProveWs::kS
   need[4] = blind ? scratch(4, m1 + 1, false) : 0;
 }
 
+// Device bytes that sizing ws for this circuit newly allocates, and those of
+// the blocks that growing buffers give back first.
+size_t ws_growth(const zk_circuit* c, const ProveWs& ws, const size_t need[ProveWs::kStreams],
+                 size_t* given_back = nullptr) {
+  const size_t m1 = c->m1, n = c->n;
+  size_t total = 0, back = 0;
+  auto grow = [&](const DeviceBuffer& b, size_t want) {
+    if (b.cap >= want) return;
+    total += want;
+    back += b.cap;
+  };
+  grow(ws.we, 32 * (m1 + 1));
+  for (const DeviceBuffer* b : {&ws.aw, &ws.bw, &ws.cw, &ws.h}) grow(*b, 32 * n);
+  for (int i = 0; i < ProveWs::kStreams; i++) grow(ws.msm[i], need[i]);
+  if (c->ctx->ntt.lmax < c->log_n) total += 2 * 16 * n;  // twiddle tables of 2^(log_n-1)
+  if (given_back) *given_back = back;
+  return total;
+}
+
 // Sizes the workspace for this circuit (buffers, MSM scratch, result copies).
-void ws_prepare(zk_circuit* c, ProveWs& ws, bool blind) {
+// The B2 MSM takes the affine accumulation (`affine`: if the caller has room
+// for it) where its scratch fits in the device's free memory beside the rest
+// of the workspace and `later` bytes that the caller goes on to allocate.
+void ws_prepare(zk_circuit* c, ProveWs& ws, bool blind, bool affine = true, size_t later = 0) {
   zk_ctx* ctx = c->ctx;
   ws.init();
   ws.nstreams = ctx->prove_streams ? ctx->prove_streams : ws.env_nstreams;
@@ -366,6 +388,12 @@ void ws_prepare(zk_circuit* c, ProveWs& ws, bool blind) {
   ws_msm_configs(c, ws.cfg);
   size_t need[ProveWs::kStreams];
   ws_scratch_needs(c, blind, ws.cfg, need);
+  size_t back = 0;
+  if (need[2] > ws.msm[2].cap &&
+      (!affine || ws_growth(c, ws, need, &back) + later > device_free_bytes() + back)) {
+    ws.cfg[2].affine = false;
+    ws_scratch_needs(c, blind, ws.cfg, need);
+  }
   const bool grow = ws.we.cap < 32 * (m1 + 1) || ws.aw.cap < 32 * n ||
                     [&] {
                       for (int i = 0; i < ProveWs::kStreams; i++)
@@ -382,10 +410,16 @@ void ws_prepare(zk_circuit* c, ProveWs& ws, bool blind) {
   ws.cw.ensure(32 * n);
   ws.h.ensure(32 * n);
   for (int i = 0; i < ProveWs::kStreams; i++) {
-    if (need[i]) ws.msm[i].ensure(need[i]);
+    if (i != 2 && need[i]) ws.msm[i].ensure(need[i]);
     ws.win[i].ensure(kMaxWindowBytes);
   }
   ctx->ntt.ensure(c->log_n, ws.st[0]);
+  // last, with what the other buffers leave
+  msm_ensure_scratch(ws.msm[2], ws.cfg[2], [&](const MsmConfig& k) {
+    ws.cfg[2] = k;
+    ws_scratch_needs(c, blind, ws.cfg, need);
+    return need[2];
+  });
 }
 
 // Witness into we = [1 || w_0 .. w_{m1-1}] on stream 0 (src/groth16.cu:1316-1326).
@@ -631,24 +665,20 @@ void note_witness(zk_circuit* c, const uint64_t* witness, bool on_device) {
 
 // Device bytes that preparing ws for this circuit would newly allocate (the
 // proof server admits a request only when that much memory is free).
-size_t ws_bytes_needed(zk_circuit* c, const ProveWs& ws, bool blind) {
+size_t ws_bytes_needed(zk_circuit* c, const ProveWs& ws, bool blind, bool affine) {
   MsmConfig cfg[ProveWs::kStreams];
   ws_msm_configs(c, cfg);
+  cfg[2].affine = affine;
   size_t need[ProveWs::kStreams];
   ws_scratch_needs(c, blind, cfg, need);
-  const size_t m1 = c->m1, n = c->n;
-  auto grow = [](const DeviceBuffer& b, size_t want) { return b.cap < want ? want : size_t(0); };
-  size_t total = grow(ws.we, 32 * (m1 + 1)) + grow(ws.aw, 32 * n) + grow(ws.bw, 32 * n) +
-                 grow(ws.cw, 32 * n) + grow(ws.h, 32 * n);
-  for (int i = 0; i < ProveWs::kStreams; i++) total += grow(ws.msm[i], need[i]);
-  if (c->ctx->ntt.lmax < c->log_n) total += 2 * 16 * n;  // twiddle tables of 2^(log_n-1)
-  return total;
+  return ws_growth(c, ws, need);
 }
 
 // Starts a proof from a host witness on ws's streams without waiting for it.
-void ws_submit(zk_circuit* c, ProveWs& ws, const uint64_t* witness, bool blind, Stager& stager) {
+void ws_submit(zk_circuit* c, ProveWs& ws, const uint64_t* witness, bool blind, bool affine,
+               Stager& stager) {
   note_witness(c, witness, false);
-  ws_prepare(c, ws, blind);
+  ws_prepare(c, ws, blind, affine);
   ws_stage(c, ws, witness, false, stager);
   ws_launch(c, ws, blind, c->ctx->use_graphs, nullptr);
   ZK_CUDA(cudaEventRecord(ws.ev_all, ws.st[0]));
@@ -664,6 +694,21 @@ void ws_collect(zk_circuit* c, ProveWs& ws, bool blind, const uint64_t* r, const
 }
 
 uint64_t next_circuit_id() { return g_circuit_ids.fetch_add(1); }
+
+void ProveWs::drop_g2_scratch() {
+  drop_graph();  // captured addresses change
+  msm[2].release();
+}
+
+void drop_g2_scratch(zk_ctx* ctx) {
+  ctx->ws.drop_g2_scratch();
+  for (auto& ws : ctx->pool) ws->drop_g2_scratch();
+  for (FusedWs& f : ctx->fused) {
+    f.drop_graphs();
+    f.g2.release();
+  }
+  ctx->msm_scratch.release();
+}
 
 void ProveWs::drop_graph() {
   for (Graph& g : graphs) cudaGraphExecDestroy(g.exec);
@@ -697,10 +742,12 @@ void prove_oneshot(zk_ctx* ctx, const BinFile& zkey, const uint64_t* witness, si
   check_job(c, witness, n_witness, false);
   note_witness(c, witness, false);
   ProveWs& ws = ctx->ws;
-  ws_prepare(c, ws, false);
+  const size_t m1 = c->m1, n = c->n, l = c->l, nc = m1 - l - 1;
+  // the points and matrices go up after the workspace: 256 bytes a variable
+  // (A, B2, C), 64 a domain element (H), 116 an entry of section 4 and its rows
+  ws_prepare(c, ws, false, true, 256 * (m1 + 1) + 96 * (size_t)n + 116 * (size_t)c->n_coefs);
   ws.flag.ensure(256);
   Stager& sg = ctx->stager;
-  const size_t m1 = c->m1, n = c->n, l = c->l, nc = m1 - l - 1;
   cudaStream_t s0 = ws.st[0];
   ZK_CUDA(cudaEventRecord(ws.ev_begin, ctx->stream));
   for (int i = 0; i < ProveWs::kStreams; i++) ZK_CUDA(cudaStreamWaitEvent(ws.st[i], ws.ev_begin, 0));

@@ -142,6 +142,18 @@ void DeviceBuffer::ensure(size_t bytes) {
   g_dev_alloc_bytes += want;
 }
 
+bool DeviceBuffer::try_ensure(size_t bytes) {
+  if (bytes <= cap && ptr) return true;
+  if (device_free_bytes() + cap < align256(bytes)) return false;
+  try {
+    ensure(bytes);
+  } catch (const Error& e) {
+    if (e.code != ZK_ENOMEM) throw;
+    return false;
+  }
+  return true;
+}
+
 void DeviceBuffer::release() {
   if (ptr) {
     if (pooled) {

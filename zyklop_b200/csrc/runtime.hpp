@@ -75,6 +75,10 @@ struct DeviceBuffer {
   DeviceBuffer& operator=(const DeviceBuffer&) = delete;
   ~DeviceBuffer() { release(); }
   void ensure(size_t bytes);
+  // ensure() where the device has room: false, with the old block kept, when
+  // its free memory does not cover the growth; false as well when the
+  // allocation fails all the same (the old block is gone then).
+  bool try_ensure(size_t bytes);
   void release();
   template <class T>
   T* as() const { return reinterpret_cast<T*>(ptr); }

@@ -26,8 +26,9 @@
 
 namespace zk {
 // prover.cu internals used by the server
-size_t ws_bytes_needed(zk_circuit* c, const ProveWs& ws, bool blind);
-void ws_submit(zk_circuit* c, ProveWs& ws, const uint64_t* witness, bool blind, Stager& stager);
+size_t ws_bytes_needed(zk_circuit* c, const ProveWs& ws, bool blind, bool affine);
+void ws_submit(zk_circuit* c, ProveWs& ws, const uint64_t* witness, bool blind, bool affine,
+               Stager& stager);
 bool ws_ready(ProveWs& ws);
 void ws_collect(zk_circuit* c, ProveWs& ws, bool blind, const uint64_t* r, const uint64_t* s,
                 uint64_t proof[32]);
@@ -90,6 +91,11 @@ struct zk_server {
       if (queue[i]->circuit->n < queue[best]->circuit->n) best = i;
     return best;
   }
+  // the G2 arenas of the slots without a proof
+  void drop_idle_scratch(const Slot* but) {
+    for (Slot& sl : slots)
+      if (&sl != but && !sl.req && sl.ws->msm[2].cap) sl.ws->drop_g2_scratch();
+  }
   void deliver(const std::shared_ptr<Request>& r, int status, const std::string& err) {
     std::lock_guard<std::mutex> g(mu);
     r->status = status;
@@ -143,9 +149,17 @@ void zk_server::run() {
         free_slot = &slots.back();
       }
       if (!free_slot) break;
+      // with the scratch of the affine G2 accumulation where there is room for
+      // it, else without, so that it never holds a request back
       size_t need = 0;
+      bool affine = true;
       try {
-        need = zk::ws_bytes_needed(r->circuit, *free_slot->ws, r->blind);
+        need = zk::ws_bytes_needed(r->circuit, *free_slot->ws, r->blind, true);
+        if (need && zk::device_free_bytes() < need + reserve) {
+          affine = false;
+          need = zk::ws_bytes_needed(r->circuit, *free_slot->ws, r->blind, false);
+          if (zk::device_free_bytes() < need + reserve) drop_idle_scratch(free_slot);
+        }
       } catch (...) {
         need = 0;
       }
@@ -170,7 +184,14 @@ void zk_server::run() {
           throw zk::Error(ZK_EWITNESS, "witness has fewer values than the circuit's nVars");
         std::lock_guard<std::mutex> g(ctx->mu);
         zk::set_current_profiler(nullptr);
-        zk::ws_submit(r->circuit, *free_slot->ws, r->witness, r->blind, stager);
+        try {
+          zk::ws_submit(r->circuit, *free_slot->ws, r->witness, r->blind, affine, stager);
+        } catch (const zk::Error& e) {
+          if (e.code != ZK_ENOMEM) throw;
+          drop_idle_scratch(nullptr);
+          zk::drop_g2_scratch(ctx);
+          zk::ws_submit(r->circuit, *free_slot->ws, r->witness, r->blind, false, stager);
+        }
         free_slot->req = r;
         busy++;
         if (busy > peak_inflight.load()) peak_inflight.store(busy);

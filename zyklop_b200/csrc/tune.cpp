@@ -33,12 +33,14 @@ int ceil_log2(size_t n) {
 int size_class(size_t n) { return n <= 1 ? 0 : (int)std::lround(std::log2((double)n)); }
 
 MsmConfig msm_config_for(const zk_ctx* ctx, bool g2, size_t n, int dist, int fixed_c) {
-  const MsmConfig& base = ctx->msm_cfg[g2 ? 1 : 0];
+  MsmConfig base = ctx->msm_cfg[g2 ? 1 : 0];
+  base.affine = ctx->affine;
   if (base.c != 0) return base;  // explicit settings win
   const auto it = ctx->tune.msm.find(std::make_tuple(g2 ? 2 : 1, size_class(n), dist, fixed_c));
   if (it == ctx->tune.msm.end()) return base;
   MsmConfig r = it->second;
   r.k1 = base.k1;
+  r.affine = base.affine;
   return r;
 }
 
@@ -114,13 +116,14 @@ void make_inputs(zk_ctx* ctx, int group, size_t n, int dist, Inputs& in) {
 
 // Median wall time of one MSM with the given settings (enqueue, copy of the
 // window sums, host combine), and its result for the cross-check.
-double time_msm(zk_ctx* ctx, const Inputs& in, const MsmConfig& cfg, int fixed_c, const void* table,
+double time_msm(zk_ctx* ctx, const Inputs& in, MsmConfig cfg, int fixed_c, const void* table,
                 DeviceBuffer& scratch, int reps, std::vector<uint64_t>& result) {
   cudaStream_t st = ctx->stream;
   const bool g2 = in.group == 2;
   const size_t n = in.n;
-  scratch.ensure(fixed_c ? msm_scratch_bytes_fixed(n, g2, fixed_c, cfg)
-                         : msm_scratch_bytes(n, g2, cfg));
+  msm_ensure_scratch(scratch, cfg, [&](const MsmConfig& k) {
+    return fixed_c ? msm_scratch_bytes_fixed(n, g2, fixed_c, k) : msm_scratch_bytes(n, g2, k);
+  });
   PinnedBuffer win;
   win.ensure(kMaxWindowBytes);
   std::vector<double> t;
@@ -198,6 +201,7 @@ TuneResult autotune_msm(zk_ctx* ctx, int group, int log_n, int dist, int fixed_c
   }
   Search s(ctx, in, fixed_c, table.ptr, reps_for(log_n));
   MsmConfig cfg = ctx->msm_cfg[g2 ? 1 : 0];
+  cfg.affine = ctx->affine;
   cfg.k0 = 64;
   cfg.chunk = 16;
   // Fixed-base MSMs start from the size defaults, which come from timing
@@ -405,7 +409,7 @@ int zk_autotune_msm(zk_ctx* ctx, int group, int log_n, int dist, int fixed_c, zk
   ZK_API_BEGIN
   ctx = zk::resolve_ctx(ctx);
   std::lock_guard<std::mutex> g(ctx->mu);
-  fill(out, zk::autotune_msm(ctx, group, log_n, dist, fixed_c));
+  zk::with_room(ctx, [&] { fill(out, zk::autotune_msm(ctx, group, log_n, dist, fixed_c)); });
   ZK_API_END
 }
 
@@ -414,7 +418,7 @@ int zk_autotune_table_c(zk_ctx* ctx, int group, int log_n, int dist, size_t max_
   ZK_API_BEGIN
   ctx = zk::resolve_ctx(ctx);
   std::lock_guard<std::mutex> g(ctx->mu);
-  fill(out, zk::autotune_table_c(ctx, group, log_n, dist, max_table_bytes));
+  zk::with_room(ctx, [&] { fill(out, zk::autotune_table_c(ctx, group, log_n, dist, max_table_bytes)); });
   ZK_API_END
 }
 
@@ -422,7 +426,7 @@ int zk_autotune_ntt(zk_ctx* ctx, int log_n, zk_tune_result* out) {
   ZK_API_BEGIN
   ctx = zk::resolve_ctx(ctx);
   std::lock_guard<std::mutex> g(ctx->mu);
-  fill(out, zk::autotune_ntt(ctx, log_n));
+  zk::with_room(ctx, [&] { fill(out, zk::autotune_ntt(ctx, log_n)); });
   ZK_API_END
 }
 
