@@ -108,3 +108,19 @@ def test_tuned_proofs_equal_oracle(api, oracle, ctx, tmp_path):
     c.set_scalar_dist(0)  # forcing the other distribution's settings changes nothing
     assert np.array_equal(c.prove(wit), want)
     c.close()
+
+
+def test_smallest_windows_on_g2(api, oracle, ctx, tmp_path):
+    """4-bit windows leave the most window sums, 65: tuning a small size tries them
+    and a proof can be told to take them"""
+    r = api.autotune_msm(2, 8, 0, ctx=ctx)
+    assert 4 <= r["c"] <= 7
+    z, w = tmp_path / "s.zkey", tmp_path / "s.wtns"
+    api.synth_circuit(z, w, 6, n_public=2, n_private_inputs=4, nnz=(1, 3), witness="uniform",
+                      seed=3)
+    want = oracle.prove(open(z, "rb").read(), open(w, "rb").read())
+    for group in (1, 2):
+        api.msm_set_config(group, c=4, ctx=ctx)
+    c = api.Circuit(z, ctx=ctx)
+    assert np.array_equal(c.prove(api.read_wtns(w)), want)
+    c.close()

@@ -14,8 +14,9 @@
 
 namespace zk {
 
-// Largest MSM result copied to the host: 2 x 64 windows of G2 XYZZ points.
-constexpr size_t kMaxWindowBytes = 2 * 64 * 256;
+// Largest MSM result copied to the host: two G2 XYZZ points for each of the
+// 256 / 4 + 1 windows of the smallest window size.
+constexpr size_t kMaxWindowBytes = 2 * 65 * 256;
 
 // Buffers and streams of one in-flight proof (reused across proofs).  A
 // context has one for single proofs and a pool for batches (a proof server
