@@ -189,8 +189,10 @@ int zk_msm_table_free(zk_msm_table* t);
 
 /* Pippenger parameters for subsequent MSMs on this context (group 1 or 2):
  * window bits c (0 = automatic), records per thread k0 (0 = by size) / k1,
- * and the fan-in `chunk` (a power of two, 0 = by size, and for fixed-base
- * MSMs by window bits) of the first bucket-reduction level.
+ * and the fan-in `chunk` (a power of two, 0 = by the number of buckets) of the
+ * first bucket-reduction level.  Large G2 MSMs (from about 2^16 points, at
+ * least six records a bucket) take an accumulation that spreads its records
+ * evenly over the device: k0 has no effect on them.
  * Replaces the reference's compile-time
  * MSM_G1_C_BITS / C_BITS and ZK_G1_* / ZK_G2_* environment knobs
  * (include/msm_g1.cuh:45-117, include/msm_g2.cuh:39-116). */
@@ -274,8 +276,10 @@ int zk_ctx_set_prove_streams(zk_ctx* ctx, int n);
  * that every candidate gives the same result, and records the fastest in the
  * context for (group, log_n, dist).  Later MSMs and proofs of that size and
  * distribution use it unless zk_msm_set_config set an explicit window.
- * Results never change.  No reference counterpart (the reference fixes its
- * window sizes and bucket tiers at compile time, include/msm_g1.cuh:714-926). */
+ * Results never change.  A fixed-base setting that does not beat the size's
+ * defaults is reported and not recorded: the size then keeps its defaults.
+ * No reference counterpart (the reference fixes its window sizes and bucket
+ * tiers at compile time, include/msm_g1.cuh:714-926). */
 typedef struct {
   int c;         /* window bits (windowed MSMs) */
   int k0;        /* sorted records per accumulation thread (bucket split threshold) */

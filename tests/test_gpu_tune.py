@@ -124,3 +124,39 @@ def test_smallest_windows_on_g2(api, oracle, ctx, tmp_path):
     c = api.Circuit(z, ctx=ctx)
     assert np.array_equal(c.prove(api.read_wtns(w)), want)
     c.close()
+
+
+def test_k0_is_not_searched_where_it_has_no_effect(api, ctx):
+    """2^17 G2 points take the affine accumulation, whose tiles k0 does not concern:
+    the setting stays the size's default, 32"""
+    r = api.autotune_msm(2, 17, 0, ctx=ctx)
+    assert r["k0"] == 32 and r["chunk"] in (2, 4, 8, 16, 32, 64)
+
+
+@pytest.mark.parametrize("fixed_c", [0, 10])
+def test_tuning_a_small_size_keeps_or_beats_its_defaults(api, ctx, fixed_c):
+    import time
+    import torch
+    lg, n = 12, 1 << 12
+    rng = np.random.default_rng(6)
+    px, py = api.mul_generator(1, rand_scalars(rng, n, False), ctx=ctx)
+    sc = rand_scalars(rng, n, False)
+    t = api.MsmTable(1, px, py, c=fixed_c, ctx=ctx) if fixed_c else None
+    run = (lambda: t.run(sc)) if fixed_c else (lambda: api.msm_g1(px, py, sc, ctx=ctx))
+
+    def best():
+        times = []
+        for _ in range(25):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            run()
+            times.append(time.perf_counter() - t0)
+        return min(times)
+    before = best()
+    r = api.autotune_msm(1, lg, 0, fixed_c=fixed_c, ctx=ctx)
+    after = best()
+    if t:
+        t.close()
+    print("defaults %.3f ms, tuned %.3f ms, %s" % (1e3 * before, 1e3 * after, r))
+    # the size's defaults are among the candidates; 6 % for the timing
+    assert after < 1.06 * before

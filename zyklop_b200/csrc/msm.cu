@@ -1459,6 +1459,27 @@ int msm_default_chunk(size_t buckets, bool fixed, bool g2) {
   return chunk;
 }
 
+namespace {
+Shape shape_for(size_t n, bool g2, const MsmConfig& cfg, int fixed_c) {
+  MsmConfig k = cfg;
+  if (fixed_c) k.c = fixed_c;
+  return make_shape(n, g2, k, fixed_c != 0);
+}
+}  // namespace
+
+MsmConfig msm_resolve(size_t n, bool g2, const MsmConfig& cfg, int fixed_c) {
+  const Shape s = shape_for(n, g2, cfg, fixed_c);
+  MsmConfig k = cfg;
+  k.c = s.c;
+  k.k0 = s.k0;
+  k.chunk = s.chunk;
+  return k;
+}
+
+bool msm_takes_affine(size_t n, bool g2, const MsmConfig& cfg, int fixed_c) {
+  return shape_for(n, g2, cfg, fixed_c).affine != 0;
+}
+
 size_t msm_scratch_bytes(size_t n, bool g2, const MsmConfig& cfg) {
   const Shape s = make_shape(n, g2, cfg);
   if (g2) return carve<fp2_t>(nullptr, s).bytes;

@@ -105,6 +105,11 @@ int msm_default_c(size_t n, bool g2);
 int msm_effective_c(size_t n, bool g2, const MsmConfig& cfg);
 int msm_default_k0(size_t n, bool fixed);
 int msm_default_chunk(size_t buckets, bool fixed, bool g2);
+// cfg with the settings it leaves to size filled in (fixed_c: the window bits of
+// a fixed-base table, 0 for a windowed MSM), and whether an MSM under cfg takes
+// the affine accumulation, which k0 does not concern.
+MsmConfig msm_resolve(size_t n, bool g2, const MsmConfig& cfg, int fixed_c);
+bool msm_takes_affine(size_t n, bool g2, const MsmConfig& cfg, int fixed_c);
 
 // Device scratch bytes one MSM of n points needs with this configuration.
 size_t msm_scratch_bytes(size_t n, bool g2, const MsmConfig& cfg);

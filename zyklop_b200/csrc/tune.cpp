@@ -200,47 +200,57 @@ TuneResult autotune_msm(zk_ctx* ctx, int group, int log_n, int dist, int fixed_c
     ZK_CUDA(cudaStreamSynchronize(ctx->stream));
   }
   Search s(ctx, in, fixed_c, table.ptr, reps_for(log_n));
+  // Both searches start from the size's defaults.
   MsmConfig cfg = ctx->msm_cfg[g2 ? 1 : 0];
   cfg.affine = ctx->affine;
-  cfg.k0 = 64;
-  cfg.chunk = 16;
-  // Fixed-base MSMs start from the size defaults, which come from timing
-  // whole proofs (overlapping MSMs), and leave them only for a clear win:
-  // a lone MSM favours shorter dependency chains and its timing is noisy.
-  double margin = 0;
-  if (fixed_c) {
-    // (within the candidates below: the shortest runs only suit small sets)
-    cfg.k0 = std::max(16, msm_default_k0(n, true));
-    cfg.chunk = std::max(4, msm_default_chunk(size_t(1) << (fixed_c - 1), true, g2));
-    margin = 0.02;
-  }
+  cfg.c = cfg.k0 = cfg.chunk = 0;
+  const MsmConfig by_size = msm_resolve(n, g2, cfg, fixed_c);
+  // Fixed-base MSMs leave the defaults, which come from timing whole proofs
+  // (overlapping MSMs), only for a clear win: a lone MSM favours shorter
+  // dependency chains and its timing is noisy.  Their candidates are the runs
+  // and chains that suit a proof's sets; where a small set's defaults are
+  // shorter than those, they are timed first and beaten or kept.
+  const double margin = fixed_c ? 0.02 : 0;
+  double default_ms = 1e30;
   if (!fixed_c) {
     // window bits first (the dominant choice), then the split threshold and
     // the reduction chunk at the best window
-    for (int c = std::max(4, log_n - 6); c <= std::min(18, log_n - 1); c++) {
-      MsmConfig k = cfg;
-      k.c = c;
-      s.trial(k);
+    for (int c = std::max(4, log_n - 6); c <= std::max(std::min(18, log_n - 1), by_size.c); c++) {
+      cfg.c = c;
+      s.trial(msm_resolve(n, g2, cfg, 0));
     }
   } else {
-    cfg.c = fixed_c;
-    s.trial(cfg);
+    MsmConfig k = by_size;
+    k.k0 = std::max(16, k.k0);
+    k.chunk = std::max(4, k.chunk);
+    if (!(k == by_size)) {
+      s.trial(by_size);
+      default_ms = s.best_ms;
+      s.best_ms = 1e30;
+    }
+    s.trial(k);
   }
-  for (int k0 : {16, 32, 64, 128, 256}) {
-    if (k0 == s.best.k0) continue;
+  const bool affine = msm_takes_affine(n, g2, s.best, fixed_c);
+  for (int k0 : {8, 16, 32, 64, 128, 256}) {
+    // the affine accumulation has no k0: its timings would be noise
+    if (k0 == s.best.k0 || affine || (fixed_c && k0 < 16)) continue;
     MsmConfig k = s.best;
     k.k0 = k0;
     s.trial(k, margin);
   }
-  for (int chunk : {4, 8, 16, 32, 64}) {
-    if (chunk == s.best.chunk) continue;
+  for (int chunk : {2, 4, 8, 16, 32, 64}) {
+    if (chunk == s.best.chunk || (fixed_c && chunk < 4)) continue;
     MsmConfig k = s.best;
     k.chunk = chunk;
     s.trial(k, margin);
   }
   MsmConfig rec = s.best;
   if (fixed_c) rec.c = 0;  // fixed-base MSMs take c from their table
-  ctx->tune.msm[std::make_tuple(group, log_n, dist, fixed_c)] = rec;
+  const auto key = std::make_tuple(group, log_n, dist, fixed_c);
+  if (s.best_ms < default_ms * (1 - margin))
+    ctx->tune.msm[key] = rec;
+  else
+    ctx->tune.msm.erase(key);  // the size keeps its defaults
   TuneResult r;
   r.cfg = s.best;
   r.table_c = fixed_c;
