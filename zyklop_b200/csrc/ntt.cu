@@ -388,15 +388,10 @@ template <bool CG, int kVecs>
 __device__ __forceinline__ void coset_elem(fr_t* (&v)[kVecs], size_t p,
                                            const fr_t* __restrict__ tw, int tw_shift, int L,
                                            const fr_t& w2n) {
+  // omega_2n^e = omega_2n^(e & 1) * omega_N^(e >> 1), and e >> 1 < N / 2 is in
+  // the table
   const size_t e = rev_bits(p, L);
-  const size_t f = e >> 1;  // omega_2n^e = omega_2n^(e & 1) * omega_N^f
-  const size_t half = L ? (size_t(1) << (L - 1)) : 1;
-  fr_t t;
-  if (f < half) {
-    t = fe_ldg<FrCfg>(tw, f << tw_shift);
-  } else {
-    t = fe_neg(fe_ldg<FrCfg>(tw, (f - half) << tw_shift));  // omega_N^(N/2) = -1
-  }
+  fr_t t = fe_ldg<FrCfg>(tw, (e >> 1) << tw_shift);
   if (e & 1) t = t * w2n;  // the upper half of the positions
 #pragma unroll
   for (int q = 0; q < kVecs; q++)
