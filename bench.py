@@ -52,7 +52,7 @@ UNIT = "proofs/s"
 # Fp multiplication (8x8 limb products lo+hi for a*b and m*p, plus m).  Both
 # are work conventions: sums of products share reductions and squares need
 # fewer limb products, so a fraction of the carry-chain probe counted this way
-# can exceed the issued one.
+# exceeds the issued one.
 FP_MULTS_PER_POINT = {"accum_g1": 176.0, "accum_g2": 528.0}
 IMAD_PER_FP_MULT = 264.0
 # what the fixed-base accumulation issues per sorted record.  A wide product is
@@ -60,10 +60,7 @@ IMAD_PER_FP_MULT = 264.0
 # XYZZ add: 6 products, 2 squares and a difference of two products with one
 # reduction.  G2, one batched affine add (large lists): a norm, 3 products of
 # the shared inversion and 2 to scale the conjugate, 2 Fp2 products (3 wide
-# products and 2 reductions each) and an Fp2 square (2 products).  Aligned
-# lo / hi pairs run as one wide multiply-add, which the carry-chain probe's
-# unpaired stream does not: issued counts reach 1.05 of it, 0.7 of the nominal
-# 64 multiply-adds per clock and SM.
+# products and 2 reductions each) and an Fp2 square (2 products).
 ISSUED_IMAD_PER_RECORD = {"accum_g1": 6 * 264 + 2 * (72 + 136) + 2 * 128 + 136,
                           "accum_g2": (2 * 72 + 136) + 5 * 264 + 2 * (3 * 128 + 2 * 136)
                           + 2 * 264}
@@ -346,8 +343,9 @@ def roofline_of(kind, rec, peak, step_ms, records_per_point=None, peak_variants=
 
 def int_peaks(L, ctx, sm_mhz):
     """The integer-pipe rates the roofline is read against (TIOP/s): the two
-    measured probes and the nominal 64 IMAD / clock / SM at the sampled SM
-    clock."""
+    measured probes (aligned lo / hi pairs of carry chains, which run as wide
+    multiply-adds, and unpaired independent ones) and the nominal 64 IMAD /
+    clock / SM at the sampled SM clock."""
     from zyklop_b200._lib import check
     out = {}
     for kind, name in ((0, "carry_chain_probe"), (1, "independent_mad_probe")):

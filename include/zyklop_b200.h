@@ -98,14 +98,14 @@ typedef struct {
 } zk_profile;
 int zk_ctx_set_profiling(zk_ctx* ctx, int on);
 int zk_ctx_profile(zk_ctx* ctx, zk_profile* out);
-/* Measured carry-chain IMAD throughput of the device (mad.lo.cc / madc.hi.cc,
- * the field multiplication's instruction mix), in 10^12 ops/s: the
- * denominator of the MSM roofline.  No reference counterpart. */
+/* Measured carry-chain IMAD throughput of the device (mad.lo.cc / madc.hi.cc
+ * on aligned register pairs, the field multiplication's instruction mix), in
+ * 10^12 ops/s: the denominator of the MSM roofline.  No reference
+ * counterpart. */
 int zk_imad_probe(zk_ctx* ctx, double* tiops);
 /* The same measurement for kind 0 (carry chains, = zk_imad_probe) or kind 1
- * (independent mad.lo / mad.hi streams without carries: the integer pipe's
- * rate when no carry flag serializes the instructions).  No reference
- * counterpart. */
+ * (independent mad.lo / mad.hi streams without carries, whose halves do not
+ * pair up: each takes its own issue slot).  No reference counterpart. */
 int zk_int_probe(zk_ctx* ctx, int kind, double* tiops);
 
 /* ---- field primitives (device pointers, n elements of 4 x u64) ----------- */
