@@ -1,7 +1,7 @@
 """The batched affine accumulation of large G2 MSMs: bases k_i G with known k_i,
 so the sum is (sum k_i s_i) G by one oracle multiplication.  Long, short and
 uneven runs, doublings, cancelling pairs, infinities among the bases, skewed
-scalars whose list is much shorter than its bound, several waves of tiles, and
+scalars whose list is much shorter than its bound, second waves of tiles, and
 the multi-instance chains of a fused batch."""
 import os
 
@@ -83,10 +83,26 @@ def test_windowed(api, oracle, kind, n, c):
     assert inf == winf and np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("kind", ["uniform", "circom"])
+def test_windowed_second_wave(api, oracle, kind):
+    """18 windows of 2^20 + 1 points: 18.9 M records, where a wave of tiles on 148 SMs
+    holds 14.5 M; the second wave reuses the scratch of the first, and runs of
+    one bucket cross from one to the other"""
+    n = (1 << 20) + 1
+    rng = np.random.default_rng(20 + len(kind))
+    ks, sc = make(rng, n, kind)
+    px, py = api.mul_generator(2, ks)
+    got, inf = api.msm_g2(px, py, sc)
+    want, winf = expect(oracle, ks, sc)
+    assert inf == winf and np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("n,c,kind", [(100003, 0, "uniform"), (100003, 14, "circom"),
-                                      (90001, 13, "few_points"), (900001, 18, "uniform")])
+                                      (90001, 13, "few_points"), (900001, 18, "uniform"),
+                                      (1000003, 18, "uniform"), (1000003, 18, "circom")])
 def test_fixed_base(api, oracle, n, c, kind):
-    """900001 points make more records than one wave of tiles holds"""
+    """900001 points (13.5 M records) are more than the 10.9 M of a wave of three
+    blocks per SM, so four run; 1000003 (15.0 M) take two waves of those"""
     rng = np.random.default_rng(n + c)
     ks, sc = make(rng, n, kind)
     px, py = api.mul_generator(2, ks)
