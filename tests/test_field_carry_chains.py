@@ -1,19 +1,22 @@
-"""The carry chains of zyklop_b200/csrc/field.cuh, restated instruction by
-instruction with PTX carry-flag semantics and checked against Python
-integers on edge and random operands (CPU only).
+"""Sums of unreduced products in zyklop_b200/csrc/field.cuh and curve_quad.cuh,
+restated word by word and checked against Python integers on edge and random
+operands (CPU only): the Fp2 product with two reductions (fp2_mul_call), the
+difference of products with one (fp_mul_sub_call), the component of an Fp2
+product that one lane of a pair forms (fp2_lane_mul_call) and the norm
+(fp2_norm_call).  The wide products, squares and reductions they are made of
+are those of test_field_pair_chains.py.
 
-The CUDA code drops carries and borrows where its comments prove they
-cannot occur (the last madc.hi of a row, the top word of a sum, the final
-borrow of a subtraction whose result is known nonnegative).  Here each of
-those places asserts that the dropped carry is zero, so a bound that does
-not hold fails the test.  Covered: mul_4x4, sqr_4x4, fe_mul_wide
-(Karatsuba over 128-bit halves), fe_sqr_wide, fe_redc, the Fp2 product
-with two reductions (fp2_mul_call) and the shared-reduction difference of
-products (fp_mul_sub_call).  The GPU parity tests check the compiled code
-itself; this test pins the arithmetic bounds those sequences rely on."""
+The CUDA code drops carries and borrows where its comments prove they cannot
+occur (the top word of a sum, the final borrow of a subtraction whose result is
+known nonnegative).  Here each of those places asserts that the dropped carry
+is zero, so a bound that does not hold fails the test.  This pins the bounds of
+the derivation; test_gpu_field_edges.py and the parity tests run the compiled
+code."""
 import random
 
 import pytest
+
+from test_field_pair_chains import limbs, mul_wide, redc_lazy, sqr_wide, val
 
 P = 21888242871839275222246405745257275088696311157297823662689037894645226208583
 R = 21888242871839275222246405745257275088548364400416034343698204186575808495617
@@ -25,14 +28,6 @@ class Cc:
 
     def __init__(self):
         self.f = 0
-
-    def mad_lo(self, a, b, c, cin=False, cout=True):
-        v = ((a * b) & M32) + c + (self.f if cin else 0)
-        return self._out(v, cout)
-
-    def mad_hi(self, a, b, c, cin=False, cout=True):
-        v = ((a * b) >> 32) + c + (self.f if cin else 0)
-        return self._out(v, cout)
 
     def add(self, a, b, cin=False, cout=True):
         return self._out(a + b + (self.f if cin else 0), cout)
@@ -53,14 +48,6 @@ class Cc:
         return v & M32
 
 
-def limbs(x, n=8):
-    return [(x >> (32 * i)) & M32 for i in range(n)]
-
-
-def val(ws):
-    return sum(w << (32 * i) for i, w in enumerate(ws))
-
-
 def chain_add(a, b):
     c = Cc()
     return [c.add(x, y, cin=i > 0, cout=i < len(a) - 1) for i, (x, y) in enumerate(zip(a, b))]
@@ -71,116 +58,10 @@ def chain_sub(a, b):
     return [c.sub(x, y, cin=i > 0, cout=i < len(a) - 1) for i, (x, y) in enumerate(zip(a, b))]
 
 
-def mul_4x4(x, y):
-    x0, x1, x2, x3 = x
-    r = [0] * 8
-    c = Cc()
-    r[0], r[1] = (x0 * y[0]) & M32, (x0 * y[0]) >> 32
-    r[2], r[3] = (x2 * y[0]) & M32, (x2 * y[0]) >> 32
-    r[1] = c.mad_lo(x1, y[0], r[1])
-    r[2] = c.mad_hi(x1, y[0], r[2], cin=True)
-    r[3] = c.mad_lo(x3, y[0], r[3], cin=True)
-    r[4] = c.mad_hi(x3, y[0], 0, cin=True, cout=False)
-    for j in (1, 2, 3):
-        yj = y[j]
-        r[j] = c.mad_lo(x0, yj, r[j])
-        r[j + 1] = c.mad_hi(x0, yj, r[j + 1], cin=True)
-        r[j + 2] = c.mad_lo(x2, yj, r[j + 2], cin=True)
-        r[j + 3] = c.mad_hi(x2, yj, r[j + 3], cin=True)
-        r[j + 4] = c.add(0, 0, cin=True, cout=False)
-        r[j + 1] = c.mad_lo(x1, yj, r[j + 1])
-        r[j + 2] = c.mad_hi(x1, yj, r[j + 2], cin=True)
-        r[j + 3] = c.mad_lo(x3, yj, r[j + 3], cin=True)
-        r[j + 4] = c.mad_hi(x3, yj, r[j + 4], cin=True, cout=False)
-    return r
-
-
-def sqr_4x4(x):
-    x0, x1, x2, x3 = x
-    r = [0] * 8
-    c = Cc()
-    r[1], r[2] = (x0 * x1) & M32, (x0 * x1) >> 32
-    r[3], r[4] = (x1 * x2) & M32, (x1 * x2) >> 32
-    r[5], r[6] = (x2 * x3) & M32, (x2 * x3) >> 32
-    r[2] = c.mad_lo(x0, x2, r[2])
-    r[3] = c.mad_hi(x0, x2, r[3], cin=True)
-    r[4] = c.mad_lo(x1, x3, r[4], cin=True)
-    r[5] = c.mad_hi(x1, x3, r[5], cin=True)
-    r[6] = c.add(r[6], 0, cin=True, cout=False)
-    r[3] = c.mad_lo(x0, x3, r[3])
-    r[4] = c.mad_hi(x0, x3, r[4], cin=True)
-    r[5] = c.add(r[5], 0, cin=True)
-    r[6] = c.add(r[6], 0, cin=True)
-    r[7] = c.add(0, 0, cin=True, cout=False)
-    r[1] = c.add(r[1], r[1])
-    for k in range(2, 7):
-        r[k] = c.add(r[k], r[k], cin=True)
-    r[7] = c.add(r[7], r[7], cin=True, cout=False)
-    r[0] = (x0 * x0) & M32
-    r[1] = c.mad_hi(x0, x0, r[1])
-    r[2] = c.mad_lo(x1, x1, r[2], cin=True)
-    r[3] = c.mad_hi(x1, x1, r[3], cin=True)
-    r[4] = c.mad_lo(x2, x2, r[4], cin=True)
-    r[5] = c.mad_hi(x2, x2, r[5], cin=True)
-    r[6] = c.mad_lo(x3, x3, r[6], cin=True)
-    r[7] = c.mad_hi(x3, x3, r[7], cin=True, cout=False)
-    return r
-
-
-def mul_wide(a, b):
-    """fe_mul_wide: middle product first, then lo, then hi."""
-    sa = chain_add(a[0:4] + [0], a[4:8] + [0])
-    sb = chain_add(b[0:4] + [0], b[4:8] + [0])
-    ca, cb = sa[4], sb[4]
-    mid = mul_4x4(sa[:4], sb[:4])
-    t = chain_add(mid[4:8] + [0], [v & ((0 - ca) & M32) for v in sb[:4]] + [0])
-    mid[4:8], m8 = t[:4], t[4]
-    t = chain_add(mid[4:8] + [m8], [v & ((0 - cb) & M32) for v in sa[:4]] + [ca & cb])
-    mid[4:8], m8 = t[:4], t[4]
-    w = mul_4x4(a[0:4], b[0:4])
-    t = chain_sub(mid + [m8], w + [0])
-    mid, m8 = t[:8], t[8]
-    T = w[0:4] + chain_add(w[4:8] + mid[4:8] + [m8], mid[0:4] + [0] * 5) + [0] * 3
-    w = mul_4x4(a[4:8], b[4:8])
-    T[8:16] = chain_add(T[8:13] + w[5:8], w[0:5] + [0, 0, 0])
-    T[4:16] = chain_sub(T[4:16], w + [0] * 4)
-    return T
-
-
-def sqr_wide(a):
-    lo, hi, x = sqr_4x4(a[0:4]), sqr_4x4(a[4:8]), mul_4x4(a[0:4], a[4:8])
-    t = chain_add(x + [0], x + [0])
-    return lo[0:4] + chain_add(lo[4:8] + hi[0:4] + hi[4:8], t[:8] + [t[8], 0, 0, 0])
-
-
 def redc(T, m):
-    """fe_redc: eight rows fold T_lo, then T_hi is added; one conditional subtraction."""
-    inv = (-pow(m, -1, 1 << 32)) % (1 << 32)
-    p = limbs(m)
-    t = T[0:8] + [0]
-    for _ in range(8):
-        q = (t[0] * inv) & M32
-        c = Cc()
-        t[0] = c.mad_lo(q, p[0], t[0])
-        t[1] = c.mad_hi(q, p[0], t[1], cin=True)
-        t[2] = c.mad_lo(q, p[2], t[2], cin=True)
-        t[3] = c.mad_hi(q, p[2], t[3], cin=True)
-        t[4] = c.mad_lo(q, p[4], t[4], cin=True)
-        t[5] = c.mad_hi(q, p[4], t[5], cin=True)
-        t[6] = c.mad_lo(q, p[6], t[6], cin=True)
-        t[7] = c.mad_hi(q, p[6], t[7], cin=True)
-        t[8] = c.add(t[8], 0, cin=True, cout=False)
-        t[1] = c.mad_lo(q, p[1], t[1])
-        t[2] = c.mad_hi(q, p[1], t[2], cin=True)
-        t[3] = c.mad_lo(q, p[3], t[3], cin=True)
-        t[4] = c.mad_hi(q, p[3], t[4], cin=True)
-        t[5] = c.mad_lo(q, p[5], t[5], cin=True)
-        t[6] = c.mad_hi(q, p[5], t[6], cin=True)
-        t[7] = c.mad_lo(q, p[7], t[7], cin=True)
-        t[8] = c.mad_hi(q, p[7], t[8], cin=True, cout=False)
-        assert t[0] == 0
-        t = t[1:9] + [0]
-    r = val(chain_add(t[0:8], T[8:16]))
+    """fe_redc: one conditional subtraction after the lazy reduction"""
+    assert val(T) < m << 256
+    r = redc_lazy(T, m)
     assert r < 2 * m, "one conditional subtraction is not enough"
     return r - m if r >= m else r
 
@@ -197,6 +78,17 @@ def fp2_mul(a0, a1, b0, b1):
 def fp_mul_sub(a, b, c, d):
     x = chain_add(mul_wide(limbs(a), limbs(b)), limbs(P * P, 16))
     return redc(chain_sub(x, mul_wide(limbs(c), limbs(d))), P)
+
+
+def fp2_lane_mul(a, ao, b0, b1, c1):
+    """one component: a b0 plus ao b1, which component 0 takes from p^2"""
+    w = mul_wide(limbs(ao), limbs(b1))
+    x = w if c1 else chain_sub(limbs(P * P, 16), w)
+    return redc(chain_add(x, mul_wide(limbs(a), limbs(b0))), P)
+
+
+def fp2_norm(a0, a1):
+    return redc(chain_add(sqr_wide(limbs(a0)), sqr_wide(limbs(a1))), P)
 
 
 def operands(m, k, seed):
@@ -227,7 +119,6 @@ def test_wide_products_up_to_2_255():
         for b in xs[:6]:
             assert val(mul_wide(limbs(a), limbs(b))) == a * b
         assert val(sqr_wide(limbs(a))) == a * a
-        assert val(sqr_4x4(limbs(a % (1 << 128), 4))) == (a % (1 << 128)) ** 2
 
 
 def test_fp2_product_two_reductions():
@@ -239,6 +130,10 @@ def test_fp2_product_two_reductions():
         c0, c1 = fp2_mul(a0, a1, b0, b1)
         assert c0 == (a0 * b0 - a1 * b1) * rinv % P
         assert c1 == (a0 * b1 + a1 * b0) * rinv % P
+        # the same product by two lanes, each with its own and its partner's part
+        assert fp2_lane_mul(a0, a1, b0, b1, False) == c0
+        assert fp2_lane_mul(a1, a0, b0, b1, True) == c1
+        assert fp2_norm(a0, a1) == (a0 * a0 + a1 * a1) * rinv % P
 
 
 def test_difference_of_products_one_reduction():
