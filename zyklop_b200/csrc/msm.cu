@@ -521,8 +521,9 @@ __global__ void __launch_bounds__(seg_threads<F>()) k_msm_accum0_queue(
 //
 // Fixed-base 2^20 points (20-bit windows, runs of 26): 5.6 ms against 7.5 ms
 // for the XYZZ accumulation, 2^18: 1.8 against 2.5.  Bound by the latency of
-// the gathers and of the scattered slots (about 700 B of DRAM traffic per
-// record), not by the multiply pipe (57 % busy).  For the same reason G1 keeps
+// the gathers and of the scattered slots (about 690 B of DRAM traffic per
+// record, 530 where the points stay in L2), not by the multiply pipe (58 %
+// busy).  For the same reason G1 keeps
 // the XYZZ accumulation, whose additions are 2.5 times cheaper: there the
 // rounds measured 2.71 against 2.70 ms.  Copying pairs to shared memory ahead
 // (cp.async) was slower: scattered 16-byte copies cost a shared-memory
@@ -1417,9 +1418,10 @@ int nearest_log2(size_t n) {
 
 // Window bits: 6 up to 2^10 points (777 points on G1: 0.30 ms, with 4 bits
 // 0.33, with 8 0.31), lg - 5 up to 2^17 (2^16 points: 11 bits 0.74 ms, 12 0.77,
-// 13 0.82), then 15 (2^20 points: 4.33 ms, 16 bits 4.34; a third shorter runs
-// of zero digits on circom-like scalars: 2.08 against 2.17), 16 from 2^22 and
-// one more per doubling beyond.  On G2, whose affine accumulation likes long
+// 13 0.82; 2^17: 12 bits 1.08, 13 1.11, 15 1.12), then 15 (2^18 points: 1.62,
+// 13 bits 1.68, 14 1.69; 2^20: 4.33 ms, 16 bits 4.34; a third shorter runs of
+// zero digits on circom-like scalars: 2.08 against 2.17), 16 from 2^22 and one
+// more per doubling beyond.  On G2, whose affine accumulation likes long
 // runs, 11 at 2^17 (2.25 ms, 12 bits 2.42) and 13 at 2^18 (3.47, 15 bits 3.68).
 int msm_default_c(size_t n, bool g2) {
   const int lg = nearest_log2(n);
@@ -1436,6 +1438,9 @@ int msm_effective_c(size_t n, bool g2, const MsmConfig& cfg) {
 // (fixed-base 2^12: 0.32 against 0.35 ms with 16), growing to 64 at 2^20
 // (windowed 2^19: 32 2.51 ms, 128 2.96, whose blocks make 1.2 waves), 128 from
 // 2^22 windowed.  Whole 2^20 proofs with tables: 64 19.0 ms, 32 19.4, 128 19.3.
+// Windowed sets around 2^18 take 16, whose shorter blocks end the last wave
+// sooner: 190000 points 1.36 ms, 32 1.39; 2^18 1.62 and 1.64; 300007 1.75 and
+// 1.76, with circom-like scalars 1.14 and 1.18 (2^18 of those: 1.07 and 1.05).
 int msm_default_k0(size_t n, bool fixed) {
   const int lg = nearest_log2(n);
   if (lg <= 13) return 8;

@@ -15,14 +15,14 @@
 //                   thread's work (skewed scalars stay balanced); buckets that
 //                   cross thread ranges leave partial sums that further levels
 //                   of the same kernel combine;
-//                      Large G2 lists first add the runs of a bucket
-//                      pairwise in affine coordinates with shared inversions
-//                      (msm_affine) and accumulate what is left;
+//                   large G2 lists first add the runs of a bucket pairwise in
+//                   affine coordinates with shared inversions (msm_affine)
+//                   and accumulate what is left;
 //   5. msm_reduce_l1 / msm_reduce_blk
 //                   sum_b (b+1) S_b per window: running sums over chunks of
 //                   buckets, then block-parallel passes (suffix scan + tree
-//                   sum over 128 partial pairs each) down to one (U, A) pair
-//                   per window;
+//                   sum over 128 partial pairs each, 64 on G2) down to one
+//                   (U, A) pair per window;
 //   6. host         A + 2^log_span U, Horner over windows (latency-bound,
 //                   done on one CPU core) and affine conversion.
 #pragma once
@@ -39,9 +39,10 @@ namespace zk {
 struct MsmConfig {
   int c = 0;          // window bits (0 = choose from n)
   int k0 = 0;         // sorted records per thread in the first accumulation level
-                      // (0 = choose from n)
+                      // (0 = choose from n; none in the affine accumulation)
   int k1 = 16;        // partial records per thread in later levels
-  int chunk = 0;      // buckets per thread in the bucket reduction (0 = choose from n)
+  int chunk = 0;      // buckets per lane group in the bucket reduction (0 = choose from
+                      // the number of buckets)
   bool affine = true; // large G2 lists: the batched affine accumulation, whose scratch
                       // is several times the rest of the arena
   bool operator==(const MsmConfig& o) const {

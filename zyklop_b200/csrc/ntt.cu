@@ -110,7 +110,7 @@ __device__ __forceinline__ fr_t fr_sub_2r(const fr_t& a, const fr_t& b) {
 }
 // x 2^-L mod r, below 2r, for x < 2r and 1 <= L <= 31: adds the multiple
 // m r (m < 2^L) that clears the low L bits and shifts; (2r + 2^L r) / 2^L <= 2r.
-// About 35 instructions against a product's 221.
+// About 35 instructions against a product's 230.
 __device__ __forceinline__ fr_t fr_div_pow2(const fr_t& x, int L) {
   const uint32_t r[8] = {FrCfg::P0, FrCfg::P1, FrCfg::P2, FrCfg::P3,
                          FrCfg::P4, FrCfg::P5, FrCfg::P6, FrCfg::P7};
