@@ -47,3 +47,14 @@ def test_inverse(inv, m):
     for x in edge + [rng.randrange(1, m) for _ in range(3000)]:
         assert inv(x, m) == pow(x, -1, m), hex(x)
     assert inv(0, m) == 0
+
+
+@pytest.mark.parametrize("m", [P, R], ids=["fp", "fr"])
+def test_unreduced_operands(inv, m):
+    """any 256 bits: the field operations take values that are not reduced"""
+    rng = random.Random(m & 0xFFF)
+    top = (1 << 256) - 1
+    for x in [m, 2 * m, 3 * m, 4 * m, 5 * m]:
+        assert inv(x, m) == 0, hex(x)
+    for x in [m + 1, 2 * m - 1, top, top - 1, 1 << 255] + [rng.getrandbits(256) for _ in range(3000)]:
+        assert inv(x, m) == pow(x, -1, m), hex(x)

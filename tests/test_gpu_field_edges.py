@@ -72,5 +72,8 @@ def test_any_256_bit_operand_beside_a_reduced_one(api, field, m):
     got = unpack(api.field_op(field, "mul", pack([a for a, _ in pairs]), pack([b for _, b in pairs])))
     assert got == [a * b * rinv % m for a, b in pairs]
     assert unpack(api.field_op(field, "decode", pack(wide))) == [a * rinv % m for a in wide]
+    rr = pow(1 << 256, 2, m)
+    assert unpack(api.field_op(field, "inv", pack(wide))) == [
+        pow(a, -1, m) * rr % m if a % m else 0 for a in wide]
     lazy = [m, 2 * m - 1] + [m + x for x in canonical(m, 7) if x]
     assert unpack(api.field_op(field, "sqr", pack(lazy))) == [a * a * rinv % m for a in lazy]

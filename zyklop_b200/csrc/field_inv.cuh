@@ -13,7 +13,7 @@
 // Range of the cofactors: |u d + v e| <= 2^30 max(|d|, |e|), and the multiple
 // of m that makes it divisible by 2^30 is at most 2^29 m in size, so a batch
 // adds at most m / 2 to the largest cofactor.  The paper's bound for inputs
-// below 2^254 is 736 steps, so 25 batches end every input with |d| < 14 m,
+// below 2^256 is 741 steps, so 25 batches end every input with |d| < 14 m,
 // far inside nine 30-bit limbs; no correction is needed before the end.
 //
 // Plain integer C++: the same code runs on the host, where a CPU test checks
@@ -131,7 +131,8 @@ ZK_HD int32_t inv_limb(const uint32_t w[8], int i) {
   return (int32_t)(x & (uint32_t)kInvMask);
 }
 
-// out = x^-1 mod m for 0 <= x < m (0 gives 0), m odd and below 2^254,
+// out = x^-1 mod m in [0, m) for any 256-bit x (a multiple of m gives 0), m an
+// odd prime below 2^254 whose low 30 bits are neither 1 nor 2^30 - 1,
 // neg_inv30 = -m^-1 mod 2^30.  Plain values, no Montgomery factor.
 ZK_HD void inv_divsteps(const uint32_t x[8], const uint32_t mw[8], uint32_t neg_inv30,
                         uint32_t out[8]) {
@@ -156,6 +157,8 @@ ZK_HD void inv_divsteps(const uint32_t x[8], const uint32_t mw[8], uint32_t neg_
     for (int i = 0; i < kInvLimbs; i++) any |= g[i];
     if (!any) break;
   }
+  // f = +-1, or +-m for a multiple of m
+  const bool unit = f[0] == 1 || f[0] == kInvMask;
   // x^-1 = sign(f) d; then into [0, m): |d| < 14 m, so d + 16 m is positive
   // and five conditional subtractions of 16 m .. m finish
   const int32_t neg = f[kInvLimbs - 1] >> 31;  // -1 when f = -1
@@ -186,7 +189,7 @@ ZK_HD void inv_divsteps(const uint32_t x[8], const uint32_t mw[8], uint32_t neg_
     uint64_t v = (uint64_t)(uint32_t)d[i] >> s;
     v |= (uint64_t)(uint32_t)d[i + 1] << (30 - s);
     if (i + 2 < kInvLimbs) v |= (uint64_t)(uint32_t)d[i + 2] << (60 - s);
-    out[k] = (uint32_t)v;
+    out[k] = unit ? (uint32_t)v : 0u;
   }
 }
 
