@@ -463,7 +463,7 @@ def run_mine(args, dist):
     assert np.array_equal(proof, reference_proof), "proofs changed with one MSM stream"
     skinds = {k: (prof.ms[i], prof.launches[i], prof.units[i]) for i, k in enumerate(Profile.KINDS)}
     # alone on one stream the fixed-base kernels issue less than the
-    # convention counts (which would read above 1): issued is the headline
+    # convention counts (which would read near or above 1): issued is the headline
     roofline_serial = {k: roofline_of(k, skinds[k], peak.value, None, wins[k], variants,
                                       headline="issued" if wins[k] else "convention")
                        for k in FP_MULTS_PER_POINT}

@@ -1,6 +1,6 @@
 """Transforms whose last pass reorders and scales (natural order, 1/N), and the
 partly reduced values between passes, bit-exact against the CPU oracle: every
-small size, pass radixes that make one to five passes, both directions, and
+small size, pass radixes that make one to four passes, both directions, and
 operands at the edges of the range."""
 import numpy as np
 import pytest
