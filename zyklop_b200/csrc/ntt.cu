@@ -463,8 +463,9 @@ void run_pass(bool dit, const PassArgs& args, int count, const fr_t* tw, int tw_
   // A launch that leaves half of the SMs idle is bound by one block's latency:
   // smaller tiles, down to one element a thread to load and store (H pipeline
   // at 2^9 / 2^12: 77 / 78 us, with full tiles 85 / 88).
-  const size_t sms = (size_t)device_sm_count();
-  while (log_g && (1 << (k + log_g)) > kPassThreads && 2 * count * (groups >> log_g) <= sms) log_g--;
+  while (log_g && (1 << (k + log_g)) > kPassThreads &&
+         2 * count * (groups >> log_g) <= (size_t)device_sm_count())
+    log_g--;
   const size_t blocks = groups >> log_g;
   const size_t smem = (size_t)8 * 4 * (size_t(1) << (k + log_g));
   dim3 grid((unsigned)blocks, count);
