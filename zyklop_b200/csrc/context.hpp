@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -105,7 +106,9 @@ struct zk_ctx {
   zk::DeviceBuffer msm_scratch;
   zk::MsmConfig msm_cfg[2];       // explicit settings (c != 0) or defaults
   zk::TuneTable tune;             // autotuned settings
-  bool affine = true;             // off while a call runs again for want of memory
+  // off while a call runs again for want of memory (a server's worker reads it
+  // without the lock when it sizes a request)
+  std::atomic<bool> affine{true};
   int scalar_dist = 0;            // distribution hint for zk_msm_g1 / g2
   zk::ProveWs ws{true};  // single proofs (ordered streams)
   std::vector<std::unique_ptr<zk::ProveWs>> pool;  // in-flight batch workspaces
